@@ -200,8 +200,8 @@ BORN_EN = 2.0
 
 
 def _born_inputs(nx, ny, rng):
-    """A Gaussian well with a weak absorbing spot, 21 points per wavelength."""
-    d = 300.0 / 2048
+    """A Gaussian well with a weak absorbing spot, 21 points per wavelength (10 on the smaller grids)."""
+    d = 300.0 / 2048 if min(nx, ny) >= 1024 else 0.32  # the box holds 24 wavelengths
     x, y = _axis(nx, d), _axis(ny, d)
     cx, cy = rng.uniform(-5, 5), rng.uniform(-5, 5)
     V = 0.3 * torch.exp(-(x[:, None] ** 2 + y[None, :] ** 2) / 4) + 0j
