@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
     const int t = threadIdx.x;
     const int n = a.n;
     C *psi = static_cast<C *>(a.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *w = static_cast<const C *>(a.w);
     const C *hs = static_cast<const C *>(a.hs);
     const C *v0 = static_cast<const C *>(a.vtab[0]);
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(M / E) k_kinetic1d_blue(BlueArgs a, double dtk
         x[e] = zero ? cmk<C>(0, 0) : cmul(psi[j], ld_c(w + j));
     }
     // FFT -> conj(. hs) -> FFT: X_k = w_k conj(result_k), |X_k| = |result_k|
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *hs = static_cast<const C *>(a.hs);
 #pragma unroll 1
     for (int ph = 0; ph < 2; ++ph) {
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(RPC *(M / E)) k_row_blue(Blue2DArgs a)
     const bool active = row < a.nx;
     const int ny = a.ny;
     C *psi = static_cast<C *>(a.psi) + (size_t)(active ? row : 0) * ny;
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *w = static_cast<const C *>(a.w);
     const C *hs = static_cast<const C *>(a.hs);
     const RowLayout<PADS> lay{line * padded<M, PADS>(M)};
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_blue(Blue2DArgs a)
     const bool active = col < a.ny;
     const int nx = a.nx, ny = a.ny;
     C *psi = static_cast<C *>(a.psi) + (active ? col : 0);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *w = static_cast<const C *>(a.w);
     const C *hs = static_cast<const C *>(a.hs);
     constexpr ColPad CP = col_pad(sizeof(C), M, W);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_blue_kinetic(Blue2DArgs a, d
         const int i = t + e * TM;
         x[e] = i < nx ? psi[(size_t)i * ny] : cmk<C>(0, 0);
     }
-    blue_dft<false, C, M, E>(x, sm, lay, CtaBarrier{}, t, static_cast<const tw_t<C> *>(a.tw),
+    blue_dft<false, C, M, E>(x, sm, lay, CtaBarrier{}, t, static_cast<const stw_t<C> *>(a.tw),
                              static_cast<const C *>(a.w), static_cast<const C *>(a.hs));
     double kin = 0, nn = 0;
     const double fy = (double)(col > ny / 2 ? ny - col : col);

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(B *G *(NY / E), born_min_blocks(B *G *(NY / E)
     const RowLayout<PADS> lay{line * LINE};
     const auto lbar = LineBarrierOf<TL, NL>::make(line);
     const CtaBarrier cbar{};
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const tw_t<C> *twx = static_cast<const tw_t<C> *>(a.tw_nx);
     const size_t base = (size_t)row * NY + t;
     const C *V = static_cast<const C *>(a.V) + base;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(W *(M / E), born_min_blocks(W *(M / E))) k_bor
     const int col = (blockIdx.x - qb * ntx) * W + c;
     C *p = static_cast<C *>(a.tmp) + ((size_t)qb * M + t) * ny + col;
     const size_t stride = (size_t)TM * ny;
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     constexpr ColPad CP = col_pad(sizeof(C), M, W, E);
     const ColLayout<W, CP.sh, CP.p> lay{c};
     const CtaBarrier bar{};
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(L / E) k_born1d(Born1DArgs a)
     const int t = threadIdx.x;
     const RowLayout<PADS> lay{0};
     const CtaBarrier bar{};
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     C *dp = static_cast<C *>(a.dpsi) + t;
     const C *p0 = static_cast<const C *>(a.psi0) + t;
     const C *V = static_cast<const C *>(a.V) + t;
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(W *(N2 / E)) k_born_fs_col(BornFsColArgs a)
     const int c = tid % W, t = tid / W;
     const int col = blockIdx.x * W + c;
     const int n1 = a.n1;
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const tw_t<C> *twn = static_cast<const tw_t<C> *>(a.tw_n);
     constexpr ColPad CP = col_pad(sizeof(C), N2, W, E);
     const ColLayout<W, CP.sh, CP.p> lay{c};
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(B *(N1 / E)) k_born_fs_row(BornFsRowArgs a)
     const int row = blockIdx.x * B + line;
     const RowLayout<PADS> lay{line * LINE};
     const auto lbar = LineBarrierOf<TL, B>::make(line);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     C *p = static_cast<C *>(a.tmp) + (size_t)row * N1 + t;
 
     C x[E];

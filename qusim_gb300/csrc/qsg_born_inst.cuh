@@ -27,11 +27,12 @@ constexpr int born_split_c(int prec, int nx, int ny)
 {
     return born_split_g0(prec, nx) * (ny / born_e(prec)) <= 512 ? born_split_g0(prec, nx) : 512 / (ny / born_e(prec));
 }
-// 2D column pass: W adjacent columns of M rows, W * M / E <= 512 threads
+// 2D column pass: W adjacent columns of M rows, W * M / E <= 512 threads (1024 for complex128
+// blocks of 4096 rows)
 constexpr int born_col_w(int prec, int m)
 {
     return prec == 1 ? (m <= 512 ? 16 : (m <= 1024 ? 8 : 4))
-                     : (m <= 256 ? 16 : (m == 512 ? 8 : (m <= 2048 ? 4 : 2)));
+                     : (m <= 256 ? 16 : (m == 512 ? 8 : (m == 1024 ? 4 : 2)));
 }
 // four-step column pass: W * N2 / E = 512 threads
 constexpr int born_fs_w(int prec, int n2) { return (prec == 1 ? 8192 : 4096) / n2; }

@@ -111,7 +111,7 @@ bool born1d_supported(int prec, uint64_t n);
 void born_fs_split(uint64_t n, int *n1, int *n2);
 
 // column-transform radix of the 2D k-space pass
-constexpr int born_col_e(int prec, int m) { return prec == 1 ? (m >= 512 ? 32 : 16) : (m >= 2048 ? 16 : 8); }
+constexpr int born_col_e(int prec, int m) { return prec == 1 ? (m >= 512 ? 32 : 16) : 8; }
 // the x split of an nx x ny grid: column blocks of <= 1024 rows (complex64) /
 // 512 (complex128), as far as a CTA of G rows of ny stays within 512 threads
 int born_split(int prec, int nx, int ny);

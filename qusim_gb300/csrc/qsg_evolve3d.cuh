@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
     const RowLayout<PADS> lay{line * LINE};
     const auto lbar = LineBarrierOf<TL, B>::make(line);
     C *psi = static_cast<C *>(a.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *kt = static_cast<const C *>(a.k);
 
     C x[E];
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(W *(L / E), min_blocks3(W *(L / E))) k3_col(Pa
     const ColLayout<W, CP.sh, CP.p> lay{c};
     const CtaBarrier bar{};
     C *psi = static_cast<C *>(a.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *kt = static_cast<const C *>(a.k);
 
     C x[E];

@@ -189,42 +189,13 @@ template <bool INV, class C> __device__ __forceinline__ void dft4(C &a0, C &a1, 
 // ---------------------------------------------------------------------------
 // Multiplication by the fixed roots of unity inside the radix-8/16 butterflies.
 //
-// complex128 uses the constants rounded once.  In complex64 the same constant
-// is applied in every transform of every step, so any error of the constant
-// itself compounds coherently; the complex64 rotations below use hi + lo
-// constants (see Roots<float2>), leaving rounding of the data.
+// complex128 transforms run in fixed point (qsg_fix.cuh).  In complex64 the same
+// constant is applied in every transform of every step, so any error of the
+// constant itself compounds coherently; the complex64 rotations below use
+// hi + lo constants (see Roots<float2>), leaving rounding of the data.
 // ---------------------------------------------------------------------------
 
 template <class C> struct Roots;
-template <> struct Roots<double2> {
-    // a * exp(-+ i th), (c, s) = (cos th, sin th)
-    template <bool INV> static __device__ __forceinline__ double2 cs(double2 a, double c, double s)
-    {
-        return INV ? cmk<double2>(a.x * c - a.y * s, a.y * c + a.x * s)
-                   : cmk<double2>(a.x * c + a.y * s, a.y * c - a.x * s);
-    }
-    static constexpr double C1 = 0.92387953251128675613, S1 = 0.38268343236508977173;
-    static constexpr double H = 0.70710678118654752440;
-    template <bool INV> static __device__ __forceinline__ double2 w16_1(double2 a) { return cs<INV>(a, C1, S1); }
-    template <bool INV> static __device__ __forceinline__ double2 w16_3(double2 a) { return cs<INV>(a, S1, C1); }
-    template <bool INV> static __device__ __forceinline__ double2 w16_9(double2 a) { return cs<INV>(a, -C1, -S1); }
-    // exp(-+ i pi/4), exp(-+ 3 i pi/4)
-    template <bool INV> static __device__ __forceinline__ double2 w8_1(double2 a)
-    {
-        return INV ? cmk<double2>((a.x - a.y) * H, (a.x + a.y) * H) : cmk<double2>((a.x + a.y) * H, (a.y - a.x) * H);
-    }
-    template <bool INV> static __device__ __forceinline__ double2 w8_3(double2 a)
-    {
-        return INV ? cmk<double2>(-(a.x + a.y) * H, (a.x - a.y) * H) : cmk<double2>((a.y - a.x) * H, -(a.x + a.y) * H);
-    }
-    // exp(-+ i r pi/16), r = 1, 3, 5, 7 (radix 32)
-    static constexpr double C16 = 0.98078528040323044913, S16 = 0.19509032201612826785;
-    static constexpr double C316 = 0.83146961230254523708, S316 = 0.55557023301960222474;
-    template <bool INV> static __device__ __forceinline__ double2 w32_1(double2 a) { return cs<INV>(a, C16, S16); }
-    template <bool INV> static __device__ __forceinline__ double2 w32_3(double2 a) { return cs<INV>(a, C316, S316); }
-    template <bool INV> static __device__ __forceinline__ double2 w32_5(double2 a) { return cs<INV>(a, S316, C316); }
-    template <bool INV> static __device__ __forceinline__ double2 w32_7(double2 a) { return cs<INV>(a, S16, C16); }
-};
 template <> struct Roots<float2> {
     // complex64: every fixed rotation multiplies by (cos th, sin th) given as
     // hi + lo float pairs (lo = float(c - hi)), as the table twiddles are.  The
@@ -613,13 +584,28 @@ template <class P> __device__ __forceinline__ const P *opaque(const P *p)
     return r;
 }
 
+}  // namespace qsg
+
+#include "qsg_fix.cuh"
+
+namespace qsg {
+
+// stage-twiddle table type of a transform: complex128 lines are transformed in
+// fixed point (qsg_fix.cuh) with fixed-point factors
+template <class C> using stw_t = std::conditional_t<std::is_same<C, double2>::value, fixw, tw_t<C>>;
+
 // Full transform of one line held in registers (natural order in and out).
-// The table's type picks the twiddle arithmetic (tw_t<C>, or float2: plain).
+// The table's type picks the twiddle arithmetic (stw_t<C>, or float2: plain).
 template <class C, int L, int E, bool INV, class Lay, class Bar, class TW>
 __device__ __forceinline__ void line_fft(C (&x)[E], C *sm, const Lay &lay, const Bar &bar, int t,
                                          const TW *__restrict__ tw)
 {
-    fft_stages<C, L, E, INV, 0>(x, sm, lay, bar, t, opaque(tw));
+    if constexpr (std::is_same<C, double2>::value) {
+        static_assert(!INV, "inverse transforms are conj(FFT(conj x))");
+        line_fft_fix<L, E>(x, sm, lay, bar, t, opaque(tw));
+    } else {
+        fft_stages<C, L, E, INV, 0>(x, sm, lay, bar, t, opaque(tw));
+    }
 }
 
 // Shared-memory index maps.  PADSHIFT adds one element of padding every
@@ -628,6 +614,10 @@ __device__ __forceinline__ void line_fft(C (&x)[E], C *sm, const Lay &lay, const
 template <int PADSHIFT> struct RowLayout {
     int base;
     __device__ __forceinline__ int operator()(int n) const { return base + n + (n >> PADSHIFT); }
+    // the first padding element of the line (no element maps to it), and whose it is
+    static constexpr bool kTile = false;
+    __device__ __forceinline__ int pad_slot() const { return base + (1 << PADSHIFT); }
+    __device__ __forceinline__ bool leader(int t) const { return t == 0; }
 };
 // column tile: element n of column c at n*W + c + (n >> SH)*P.  The pad is a
 // function of the row index only, so every address of a thread is a base plus
@@ -637,6 +627,11 @@ template <int PADSHIFT> struct RowLayout {
 template <int W, int SH, int P> struct ColLayout {
     int c;
     __device__ __forceinline__ int operator()(int n) const { return n * W + c + (n >> SH) * P; }
+    // the first padding element of the tile (shared by its columns)
+    static_assert(P >= 1, "padded tiles only");
+    static constexpr bool kTile = true;
+    __device__ __forceinline__ int pad_slot() const { return (1 << SH) * W; }
+    __device__ __forceinline__ bool leader(int t) const { return t == 0 && c == 0; }
 };
 struct ColPad {
     int sh, p;

@@ -1,0 +1,338 @@
+// qsg_fix.cuh -- complex128 line transforms in 64-bit block fixed point.
+//
+// GB300 runs FP64 at 2 instructions per clock and SM (measured: dfma 2.0,
+// dadd 1.7, conversions to and from double 2.0), but 64-bit integer adds at 59
+// and 32 x 32 + 64 multiply-adds (IMAD.WIDE) at 25-32.  A transform is mostly
+// additions, so complex128 lines are transformed on integers: the line's values
+// become v * 2^ex with one exponent per line (per tile for column tiles), the
+// butterflies add 64-bit integers exactly, the twiddle products round to the
+// last place, and the line goes back to double at the end.
+//
+// Precision.  The largest component of a line is kept between 2^57 and 2^61
+// units of the fixed point (re-scaled after a stage by the largest magnitude the
+// stage left, a reduction that rides on the exchange's barrier), so every
+// rounding is at most 2^-57 of the line's largest value, where a double's is
+// 2^-53 of each value.  An FFT's error is relative to the line's norm in either
+// arithmetic; measured figures stand at line_fft_fix.
+//
+// A unit-modulus factor w is stored as {re hi, re lo, im hi, im lo}: hi =
+// round(w 2^30), lo = the rest at 2^-62, so w is held to 2^-63.
+#pragma once
+
+namespace qsg {
+
+struct Fix {
+    long long x, y;
+};
+// table entry of a unit-modulus factor: {re hi, re lo, im hi, im lo}
+using fixw = int4;
+
+template <> struct RealOf<Fix> { using type = long long; };
+
+__device__ __forceinline__ int fix_hi(long long v) { return (int)(v >> 32); }
+__device__ __forceinline__ int fix_lo(long long v) { return (int)v; }
+// v = fix_hir(v) 2^32 + (signed) fix_lo(v): the high word rounded up where the low word, taken as signed, is negative
+__device__ __forceinline__ int fix_hir(long long v) { return fix_hi(v) + (int)((unsigned)fix_lo(v) >> 31); }
+// c + a b in 64 bits (IMAD.WIDE)
+__device__ __forceinline__ long long fix_mad(int a, int b, long long c) { return (long long)a * b + c; }
+
+// a w / 4 for |a.x|, |a.y| < 2^61.  With a = h 2^32 + l and w = wh 2^-30 + wl 2^-62,
+// a w / 4 = h wh + (h wl + l wh) 2^-32 (+ l wl 2^-64, left out: below half a unit);
+// the middle sum is rounded (the 2^31), so the product is unbiased.
+__device__ __forceinline__ Fix fix_twmul(Fix a, fixw w)
+{
+    const int xh = fix_hir(a.x), xl = fix_lo(a.x), yh = fix_hir(a.y), yl = fix_lo(a.y);
+    const int nh = -w.z, nl = -w.w;
+    long long tr = fix_mad(xh, w.y, 1ll << 31), ti = fix_mad(xh, w.w, 1ll << 31);
+    tr = fix_mad(xl, w.x, tr);
+    ti = fix_mad(xl, w.z, ti);
+    tr = fix_mad(yh, nl, tr);
+    ti = fix_mad(yh, w.y, ti);
+    tr = fix_mad(yl, nh, tr);
+    ti = fix_mad(yl, w.x, ti);
+    Fix r;
+    r.x = fix_mad(yh, nh, fix_mad(xh, w.x, tr >> 32));
+    r.y = fix_mad(yh, w.x, fix_mad(xh, w.z, ti >> 32));
+    return r;
+}
+
+// u / sqrt(2), to one unit
+__device__ __forceinline__ long long fix_h(long long u)
+{
+    constexpr int HH = 1518500250, HL = -51432894;  // 2^31 / sqrt(2) = HH + HL 2^-32
+    const int h = fix_hir(u), l = fix_lo(u);
+    const long long t = fix_mad(l, HH, fix_mad(h, HL, 1ll << 31));
+    const long long a = fix_mad(h, HH, t >> 32);
+    return a + a;
+}
+
+template <> struct Roots<Fix> {
+    template <bool INV> static __device__ __forceinline__ Fix w8_1(Fix a)
+    {
+        return INV ? Fix{fix_h(a.x - a.y), fix_h(a.x + a.y)} : Fix{fix_h(a.x + a.y), fix_h(a.y - a.x)};
+    }
+    template <bool INV> static __device__ __forceinline__ Fix w8_3(Fix a)
+    {
+        return INV ? Fix{-fix_h(a.x + a.y), fix_h(a.x - a.y)} : Fix{fix_h(a.y - a.x), -fix_h(a.x + a.y)};
+    }
+};
+template <> struct RootsOf<Fix, fixw> { using type = Roots<Fix>; };
+
+// OR of the magnitudes' high words over a thread's slots (its bit length bounds every component's)
+template <int E> __device__ __forceinline__ unsigned fix_or(const Fix (&v)[E])
+{
+    unsigned m = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int a = fix_hi(v[e].x), b = fix_hi(v[e].y);
+        m |= (unsigned)(a ^ (a >> 31));
+        m |= (unsigned)(b ^ (b >> 31));
+    }
+    return m;
+}
+
+// Reduction over the threads that share a layout's exponent (a line of TL
+// threads; a column tile: the CTA).  Lines within a warp shuffle; larger groups
+// OR / MAX one word per warp into the padding words of their exchange buffer.
+// `put` runs before a barrier of the group, `get` after it.  OP 0: OR, 1: max.
+template <int TL, class Lay, int OP> struct FixReduce {
+    static constexpr bool WARP = !Lay::kTile && TL <= 32;
+    static __device__ __forceinline__ unsigned op(unsigned a, unsigned b) { return OP ? (a > b ? a : b) : (a | b); }
+    static __device__ __forceinline__ unsigned put(unsigned v, unsigned *word)
+    {
+        if constexpr (WARP) {
+            const unsigned lane = threadIdx.x & 31;
+            const unsigned mask = TL == 32 ? 0xffffffffu : ((1u << (TL & 31)) - 1u) << (lane & ~(unsigned)(TL - 1));
+#pragma unroll
+            for (int o = TL / 2; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(mask, v, o));
+            return v;
+        } else {
+            v = OP ? __reduce_max_sync(0xffffffffu, v) : __reduce_or_sync(0xffffffffu, v);
+            if ((threadIdx.x & 31) == 0) {
+                if (OP)
+                    atomicMax(word, v);
+                else
+                    atomicOr(word, v);
+            }
+            return v;
+        }
+    }
+    static __device__ __forceinline__ unsigned get(unsigned v, const unsigned *word)
+    {
+        return WARP ? v : *const_cast<const volatile unsigned *>(word);
+    }
+};
+
+// the double d as units of 2^(emax - 1023 - 58): its 53-bit significand from bit 58 down,
+// shifted by the distance of its exponent from emax (magnitude bits below the unit dropped)
+__device__ __forceinline__ long long fix_from(double d, int emax)
+{
+    const int hi = __double2hiint(d);
+    const unsigned lo = (unsigned)__double2loint(d);
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const unsigned long long m = ((unsigned long long)mh << 32 | lo) << 6;
+    int sh = emax - e;
+    sh = sh > 63 ? 63 : sh;
+    const long long v = (long long)(m >> sh);
+    const long long s = (long long)(hi >> 31);
+    return (v ^ s) - s;
+}
+
+// v 2^ex as a double, rounded to nearest; ex keeps every result in the normal range (see fix_out)
+__device__ __forceinline__ double fix_to(long long v, int ex)
+{
+    const int s = fix_hi(v) >> 31;
+    const long long sl = s;
+    const unsigned long long a = (unsigned long long)((v ^ sl) - sl);
+    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+    const int lz = __clz(ah ? (int)ah : (int)al) + (ah ? 0 : 32);  // 1 .. 64
+    const unsigned long long m = ((a << (lz - 1)) + 0x200ull) >> 10;  // the leading one at bit 52 (53 on a carry)
+    // biased exponent - 1: the leading one adds the 1 (and a carry one more)
+    const int eb = a ? ex + (63 - lz) + 1022 : 0;
+    return __hiloint2double((int)(((unsigned)(m >> 32) + ((unsigned)eb << 20)) | ((unsigned)s & 0x80000000u)),
+                            (int)(unsigned)m);
+}
+
+// double line -> fixed point; returns the exponent (value = v 2^ex), and whether the line is finite.
+// mx: the largest high word (sign cleared) of the line.  A line near the bottom of the range
+// is scaled by an exact power of two first, which also makes its subnormal values normal.
+template <int E> __device__ __forceinline__ int fix_in(double2 (&x)[E], Fix (&v)[E], unsigned mx, bool *finite)
+{
+    int emax = (int)(mx >> 20), up = 0;
+    *finite = emax != 0x7ff;
+    if (emax < 64) {
+        up = 200;
+        emax += up;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            x[e].x *= 0x1p200;
+            x[e].y *= 0x1p200;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        v[e].x = fix_from(x[e].x, emax);
+        v[e].y = fix_from(x[e].y, emax);
+    }
+    return emax - up - 1023 - 58;
+}
+
+template <int E> __device__ __forceinline__ unsigned fix_absmax(const double2 (&x)[E])
+{
+    unsigned m = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const unsigned a = (unsigned)__double2hiint(x[e].x) & 0x7fffffffu, b = (unsigned)__double2hiint(x[e].y) & 0x7fffffffu;
+        m = a > m ? a : m;
+        m = b > m ? b : m;
+    }
+    return m;
+}
+
+// fixed point -> double.  Exponents whose results could leave the normal range
+// go through a second, exact power of two; a line that held an infinity or a NaN
+// becomes NaN throughout, as its transform is.
+template <int E> __device__ __forceinline__ void fix_out(const Fix (&v)[E], double2 (&x)[E], int ex, bool finite)
+{
+    const bool tiny = ex < -900, huge = ex > 900;
+    const int e2 = tiny ? ex + 400 : huge ? ex - 400 : ex;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        x[e].x = fix_to(v[e].x, e2);
+        x[e].y = fix_to(v[e].y, e2);
+    }
+    if (tiny || huge || !finite) {
+        const double sc = !finite ? __hiloint2double(0x7ff80000, 0) : tiny ? 0x1p-400 : 0x1p400;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            x[e].x *= sc;
+            x[e].y *= sc;
+        }
+    }
+}
+
+// Scale a line so that every component is below 2^61 units and the largest is
+// not far below: m is the OR of the magnitudes' high words.
+template <int E> __device__ __forceinline__ void fix_norm(Fix (&v)[E], unsigned m, int &ex)
+{
+    const int top = 31 - __clz((int)m);  // bit length - 1 of the high words (-1: all below 2^32)
+    if (top > 28) {
+        const int r = top - 28;  // 1 or 2
+        const long long half = 1ll << (r - 1);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            v[e].x = (v[e].x + half) >> r;
+            v[e].y = (v[e].y + half) >> r;
+        }
+        ex += r;
+    } else if (top < 25) {
+        const int l = 28 - top;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            v[e].x <<= l;
+            v[e].y <<= l;
+        }
+        ex -= l;
+    }
+}
+
+// One Stockham stage on fixed point (fft_stage's data movement); ex follows the scale.
+template <int L, int E, int S, class Lay, class Bar>
+__device__ __forceinline__ void fix_stage(Fix (&x)[E], Fix *sm, unsigned *words, const Lay &lay, const Bar &bar, int t,
+                                          const fixw *__restrict__ tw, int &ex)
+{
+    using P = Plan<L, E>;
+    constexpr int RL = P::radix_log(S);
+    constexpr int R = 1 << RL;
+    static_assert(R <= 8, "radix 2, 4 or 8: the head room above 2^61 / 4 units is 8 sqrt(2)");
+    constexpr int PL = P::p_log(S);
+    constexpr int PP = 1 << PL;
+    constexpr int J = E / R;
+    constexpr int TL = P::TL;
+    constexpr int TWO = P::tw_offset(S);
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        Fix v[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = x[j + q * J];
+        if constexpr (PP > 1) {
+            const int k = (t + j * TL) & (PP - 1);
+            v[0].x = (v[0].x + 2) >> 2;
+            v[0].y = (v[0].y + 2) >> 2;
+#pragma unroll
+            for (int q = 1; q < R; ++q) v[q] = fix_twmul(v[q], __ldg(&tw[TWO + (q - 1) * PP + k]));
+        }
+        dft<R, false, Fix, fixw>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[j + q * J] = v[q];
+    }
+    if constexpr (PP > 1) ex += 2;
+    if constexpr (S + 1 < P::NST) {
+        using Red = FixReduce<TL, Lay, 0>;
+        constexpr int WD = 1 + (S & 1);  // this exchange's word (zeroed in the exchange before)
+        const unsigned m = Red::put(fix_or(x), words + WD);
+        bar();  // every reader of the previous stage is done with the buffer
+        if constexpr (!Red::WARP) {
+            if (lay.leader(t)) words[3 - WD] = 0;  // the next exchange's word
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int b = t + j * TL;
+            const int k = b & (PP - 1);
+            const int o = ((b - k) << RL) + k;
+#pragma unroll
+            for (int q = 0; q < R; ++q) sm[lay(o + q * PP)] = x[j + q * J];
+        }
+        bar();
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e] = sm[lay(t + e * TL)];
+        fix_norm(x, Red::get(m, words + WD), ex);
+    }
+}
+
+template <int L, int E, int S, class Lay, class Bar>
+__device__ __forceinline__ void fix_stages(Fix (&x)[E], Fix *sm, unsigned *words, const Lay &lay, const Bar &bar, int t,
+                                           const fixw *__restrict__ tw, int &ex)
+{
+    if constexpr (S < Plan<L, E>::NST) {
+        fix_stage<L, E, S>(x, sm, words, lay, bar, t, tw, ex);
+        fix_stages<L, E, S + 1>(x, sm, words, lay, bar, t, tw, ex);
+    }
+}
+
+// Forward transform of a complex128 line (line_fft's contract).
+// Measured against FP64 butterflies (whole calls): 1024^2 O4 1035 -> 332 us a
+// step, a 1000-site wall 595 -> 204 us, 131072-site lines 82 -> 41 us, 450 x 700
+// 668 -> 247 us; error against 64-bit references 1.3e-14 -> 1.2e-14, 2.0e-14 ->
+// 1.3e-14, 1.2e-14 -> 1.1e-14, 8e-15 -> 4e-15 on the same runs.
+template <int L, int E, class Lay, class Bar>
+__device__ __forceinline__ void line_fft_fix(double2 (&x)[E], double2 *smd, const Lay &lay, const Bar &bar, int t,
+                                             const fixw *__restrict__ tw)
+{
+    static_assert(sizeof(Fix) == sizeof(double2), "the exchange buffer is shared");
+    static_assert(Plan<L, E>::NST >= 2, "a line has at least one exchange");
+    Fix *sm = reinterpret_cast<Fix *>(smd);
+    unsigned *words = reinterpret_cast<unsigned *>(smd + lay.pad_slot());
+    using Red = FixReduce<L / E, Lay, 1>;
+    unsigned mx = fix_absmax(x);
+    if constexpr (Red::WARP) {
+        mx = Red::put(mx, words);
+    } else {
+        // word 0's last readers are behind an exchange's barrier of the transform before; word 1
+        // (this transform's first exchange's) may still be read until every thread is here
+        if (lay.leader(t)) words[0] = 0;
+        bar();
+        Red::put(mx, words);
+        if (lay.leader(t)) words[1] = 0;
+        bar();
+        mx = Red::get(mx, words);
+    }
+    Fix v[E];
+    bool finite;
+    int ex = fix_in(x, v, mx, &finite);
+    fix_stages<L, E, 0>(v, sm, words, lay, bar, t, tw, ex);
+    fix_out(v, x, ex, finite);
+}
+
+}  // namespace qsg

@@ -116,8 +116,20 @@ inline int dev_alloc(qsg_ctx *ctx, size_t bytes, void **p, size_t *acct, bool bu
 // twiddle table entry: complex128 {re, im}; complex64 {hi.re, hi.im, lo.re, lo.im}
 // with hi = float(v), lo = float(v - hi)
 // table precision codes: 0 complex128, 1 complex64 hi + lo (float4),
-// 2 complex64 plain (float2, each factor rounded once)
+// 2 complex64 plain (float2, each factor rounded once), 3 fixed point (fixw, qsg_fix.cuh)
 inline size_t twsize(int prec) { return prec == 2 ? 8 : 16; }
+
+// |v| <= 1 as hi 2^-30 + lo 2^-62 (lo kept within +-(2^31 - 1), so both words can be negated)
+inline void put_fixed(long double v, int32_t *hi, int32_t *lo)
+{
+    const long double s = v * 1073741824.0L;
+    const long double h = roundl(s);
+    long double l = roundl((s - h) * 4294967296.0L);
+    if (l > 2147483647.0L) l = 2147483647.0L;
+    if (l < -2147483647.0L) l = -2147483647.0L;
+    *hi = (int32_t)h;
+    *lo = (int32_t)l;
+}
 
 inline void put_twiddle(int prec, unsigned char *dst, long double re, long double im)
 {
@@ -128,13 +140,18 @@ inline void put_twiddle(int prec, unsigned char *dst, long double re, long doubl
         const float hr = (float)re, hi = (float)im;
         float v[4] = {hr, hi, (float)(re - (long double)hr), (float)(im - (long double)hi)};
         std::memcpy(dst, v, 16);
+    } else if (prec == 3) {
+        int32_t v[4];
+        put_fixed(re, &v[0], &v[1]);
+        put_fixed(im, &v[2], &v[3]);
+        std::memcpy(dst, v, 16);
     } else {
         double v[2] = {(double)re, (double)im};
         std::memcpy(dst, v, 16);
     }
 }
 
-// stage-major twiddles of qsg::Plan<L, E>, from long double
+// stage-major twiddles of qsg::Plan<L, E>, from long double (complex128: fixed-point factors)
 inline int get_twiddles(qsg_ctx *ctx, int prec, int L, int E, const void **out)
 {
     auto key = std::make_tuple(prec, L, E);
@@ -159,7 +176,7 @@ inline int get_twiddles(qsg_ctx *ctx, int prec, int L, int E, const void **out)
         off += (R - 1) * P;
     }
     std::vector<unsigned char> host(size * twsize(prec));
-    for (int i = 0; i < size; ++i) put_twiddle(prec, &host[i * twsize(prec)], re[i], im[i]);
+    for (int i = 0; i < size; ++i) put_twiddle(prec == 0 ? 3 : prec, &host[i * twsize(prec)], re[i], im[i]);
     void *d = nullptr;
     int rc = dev_alloc(ctx, host.size(), &d, nullptr);
     if (rc) return rc;

@@ -171,12 +171,14 @@ struct RowPassArgs {
 // The body, for a compile-time in_split (see k_row_pass).
 // the twiddle table type of a pass: PL (complex64 only) selects plain float2 tables
 template <class C, bool PL> using pass_tw_t = std::conditional_t<PL, float2, tw_t<C>>;
+template <class C, bool PL> using pass_stw_t = std::conditional_t<PL, float2, stw_t<C>>;
 
 template <class T, int NY, int E, int G, int B, int RS, bool IN, bool PL>
 __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned char *smraw, double *red)
 {
     using C = cplx_t<T>;
     using TW = pass_tw_t<C, PL>;
+    using STW = pass_stw_t<C, PL>;
     static_assert(!PL || sizeof(C) == 8, "plain twiddles are a complex64 form");
     using P = Plan<NY, E>;
     constexpr int TL = P::TL;
@@ -195,7 +197,7 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
     const int t = tid - grp * TL;
     const C *in = static_cast<const C *>(a.in);
     C *out = static_cast<C *>(a.out);
-    const TW *tw = static_cast<const TW *>(a.tw_row);
+    const STW *tw = static_cast<const STW *>(a.tw_row);
     const TW *twx = static_cast<const TW *>(a.tw_nx);
     const C *vt = static_cast<const C *>(a.vtab);
     const CtaBarrier cbar{};
@@ -429,7 +431,7 @@ template <class T, int M, int E, int W, bool PL = false>
 __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : 1) k_col_pass(ColPassArgs a)
 {
     using C = cplx_t<T>;
-    using TW = pass_tw_t<C, PL>;
+    using TW = pass_stw_t<C, PL>;
     using P = Plan<M, E>;
     constexpr int TM = P::TL;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(L / E) k_kinetic1d(const void *psi_, const voi
     C x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = psi[t + e * TL];
-    line_fft<C, L, E, false>(x, sm, RowLayout<PADS>{0}, CtaBarrier{}, t, static_cast<const tw_t<C> *>(tw_));
+    line_fft<C, L, E, false>(x, sm, RowLayout<PADS>{0}, CtaBarrier{}, t, static_cast<const stw_t<C> *>(tw_));
     double k = 0, nn = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_kinetic(ColPassArgs a, doubl
     for (int e = 0; e < E; ++e) x[e] = psi[base + (size_t)(t + e * TM) * ny];
     constexpr ColPad CP = col_pad(sizeof(C), M, W);
     line_fft<C, M, E, false>(x, sm, ColLayout<W, CP.sh, CP.p>{c}, CtaBarrier{}, t,
-                             static_cast<const tw_t<C> *>(a.tw_col));
+                             static_cast<const stw_t<C> *>(a.tw_col));
     const double fy = double(col > ny / 2 ? ny - col : col);
     double k = 0, nn = 0;
 #pragma unroll
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(W *(N2 / E), (W * (N2 / E) <= 256 && sizeof(T)
     const int col = blockIdx.x * W + c;
     const int n1 = a.n1;
     C *psi = static_cast<C *>(in.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw_col);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw_col);
     const tw_t<C> *twn = static_cast<const tw_t<C> *>(a.tw_n);
     constexpr ColPad CP = col_pad(sizeof(C), N2, W);
     const ColLayout<W, CP.sh, CP.p> lay{c};
@@ -792,7 +794,7 @@ __global__ void __launch_bounds__(B *(N1 / E)) k_fs_row(FsRowArgs a)
     const RowLayout<PADS> lay{line * LINE};
     const auto lbar = LineBarrierOf<TL, B>::make(line);
     C *psi = static_cast<C *>(in.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw_row);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw_row);
     const size_t base = (size_t)row * N1 + t;
 
     C x[E];
@@ -844,7 +846,7 @@ __global__ void __launch_bounds__(B *(N1 / E)) k_fs_row_kinetic(FsRowArgs a, int
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = psi[(size_t)row * N1 + t + e * TL];
     line_fft<C, N1, E, false>(x, sm, RowLayout<PADS>{line * LINE}, CtaBarrier{}, t,
-                              static_cast<const tw_t<C> *>(a.tw_row));
+                              static_cast<const stw_t<C> *>(a.tw_row));
     const long n = (long)N1 * n2;
     double k = 0, nn = 0;
 #pragma unroll
@@ -893,7 +895,7 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
     const bool active = line < count;
     const FsInst in = a.inst[active ? idx : first];
     C *psi = static_cast<C *>(in.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(twp);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(twp);
     const C *v0 = static_cast<const C *>(in.vtab[0]);
     const C *v1 = static_cast<const C *>(in.vtab[1]);
     const C *k0 = static_cast<const C *>(in.ktab[0]);
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
     const int t = threadIdx.x;
     const FsInst in = a.inst[blockIdx.x];
     C *psi = static_cast<C *>(in.psi);
-    const tw_t<C> *tw = static_cast<const tw_t<C> *>(a.tw);
+    const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
     const C *v0 = static_cast<const C *>(in.vtab[0]);
     const C *v1 = static_cast<const C *>(in.vtab[1]);
     const C *k0 = static_cast<const C *>(in.ktab[0]);
@@ -1168,7 +1170,7 @@ __global__ void __launch_bounds__(L2 / E) k_kinetic1d_wall(const void *psi_, con
     odd_extend<C, L2, E>(x, sm, lay, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
-    line_fft<C, L2, E, false>(x, sm, lay, CtaBarrier{}, t, static_cast<const tw_t<C> *>(tw_));
+    line_fft<C, L2, E, false>(x, sm, lay, CtaBarrier{}, t, static_cast<const stw_t<C> *>(tw_));
     double k = 0, nn = 0;
 #pragma unroll
     for (int e = 0; e < H; ++e) {

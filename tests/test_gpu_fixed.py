@@ -1,0 +1,89 @@
+"""The fixed-point line transforms of the complex128 path (csrc/qsg_fix.cuh) at
+the edges of their scaling: lines far from 1 in magnitude, impulses and
+constants (the extremes of peak against norm), zero and non-finite lines,
+neighbouring columns of very different size.  The bar is the path's own,
+relative L2 <= 1e-12 against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+@pytest.fixture(scope="module")
+def qsg():
+    import qusim_gb300 as q
+    q.load()
+    return q
+
+
+@pytest.fixture(scope="module")
+def ctx(qsg):
+    return qsg.Context(0)
+
+
+def rel_l2(a, b):
+    return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
+
+
+def line(n, kind, seed=0):
+    rng = np.random.default_rng(seed)
+    if kind == "impulse":
+        psi = np.zeros(n, np.complex128)
+        psi[n // 3] = 1.0 - 0.5j
+    elif kind == "constant":
+        psi = np.full(n, 0.75 + 0.25j)
+    else:
+        psi = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    V = rng.uniform(-1, 1, n)
+    return psi, V
+
+
+# 64: lines of 8 threads; 256: one warp; 512: two warps; 4096: the longest; 1000, 3000: Bluestein;
+# 8192, 32768: four-step
+@pytest.mark.parametrize("n", [64, 256, 512, 4096, 1000, 3000, 8192, 32768])
+@pytest.mark.parametrize("kind", ["impulse", "constant", "noise"])
+def test_lines_of_any_scale_vs_oracle(qsg, ctx, oracle, n, kind):
+    psi, V = line(n, kind)
+    ref = oracle.evolve1d(psi, V, 0.1, 0.01, 3, order=4)
+    # powers of two are exact, so the scaled state's result is the scaled result; near 2^-1000 the
+    # smallest components are subnormal (2^-1074 against 2^-1000)
+    for k in (0, -1000, -400, 900):
+        inst = qsg.Instance.create_1d(ctx, np.ldexp(psi.view(np.float64), k).view(np.complex128), V, 0.1, 0.01,
+                                      order=4)
+        inst.step(3)
+        got = np.ldexp(inst.get_psi().view(np.float64), -k).view(np.complex128)
+        assert rel_l2(got, ref) <= TOL, k
+        inst.close()
+
+
+@pytest.mark.parametrize("n", [64, 4096, 1000, 8192])
+def test_zero_line_stays_zero(qsg, ctx, n):
+    _, V = line(n, "noise")
+    inst = qsg.Instance.create_1d(ctx, np.zeros(n, np.complex128), V, 0.1, 0.01, order=2)
+    inst.step(2)
+    assert np.all(inst.get_psi() == 0)
+
+
+@pytest.mark.parametrize("n", [64, 4096, 8192])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_non_finite_site_spreads_over_the_line(qsg, ctx, n, bad):
+    psi, V = line(n, "noise")
+    psi[n // 5] = bad
+    inst = qsg.Instance.create_1d(ctx, psi, V, 0.1, 0.01, order=2)
+    inst.step(1)
+    assert not np.isfinite(inst.get_psi()).any()
+
+
+@pytest.mark.parametrize("shape", [(128, 128), (256, 1024), (4096, 128), (100, 45)])
+def test_columns_of_very_different_size_vs_oracle(qsg, ctx, oracle, shape):
+    nx, ny = shape
+    rng = np.random.default_rng(1)
+    psi = (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)) * np.exp(-40.0 * (np.arange(ny) % 7))[None, :]
+    psi *= np.exp(-30.0 * (np.arange(nx) % 5))[:, None]
+    V = rng.uniform(-1, 1, shape)
+    ref = oracle.evolve2d(psi, V, 0.1, 0.1, 0.01, 2, order=4)
+    inst = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, 0.01, order=4)
+    inst.step(2)
+    assert rel_l2(inst.get_psi(), ref) <= TOL
