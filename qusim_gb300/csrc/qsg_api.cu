@@ -170,12 +170,18 @@ struct qsg_inst {
     unsigned *err = nullptr;
     unsigned err_seen = 0;
     bool lost = false;
+    // complex128 passes that apply their phase factors in fixed point (real time
+    // steps): the phase tables hold fixed-point factors
+    bool fx = false;
     std::vector<void *> allocs;
     size_t bytes = 0;
 };
 
 namespace {
 
+
+// form of the instance's phase tables (qsg_aux.h)
+int tab_prec(const qsg_inst *in) { return in->fx ? 3 : in->prec; }
 
 int inst_alloc(qsg_inst *in, size_t bytes, void **p)
 {
@@ -444,6 +450,7 @@ int row_pass(qsg_inst *in, bool is, bool os, const void *v, bool vtwice, double 
     a.vtwice = vtwice ? 1 : 0;
     a.vdiff = vdiff ? 1 : 0;
     a.plain = vdiff ? 1 : 0;
+    a.fx = in->fx ? 1 : 0;
     a.tw_row = vdiff ? in->tw_row_p : in->tw_row;
     a.tw_nx = vdiff ? in->tw_nx_p : in->tw_nx;
     a.partials = partials;
@@ -475,6 +482,7 @@ int col_pass(qsg_inst *in, int d, double *partials = nullptr, bool first = false
     a.plain = momentum(in) && !(first || whole || inv_only) ? 1 : 0;
     a.kx = in->kx[d];
     a.ky = in->ky[d];
+    a.fx = in->fx ? 1 : 0;
     a.k2d = in->ktab[d];
     a.tw_col = a.plain ? in->tw_col_p : in->tw_col;
     a.nx = in->nx;
@@ -1172,8 +1180,9 @@ int build_tables(qsg_inst *in)
     for (int k = 0; k < ntab; ++k) {
         // ExpV coefficient -i/hbar * dt * c (SplittingMethod1D.cpp:87, SplittingMethod2D.cpp:43-50)
         const cd f = (-I / in->hbar) * in->dt * vc[k];
-        if ((rc = inst_alloc(in, in->n * cs, &in->vtab[k]))) return rc;
-        QSG_CUDA(qsg::launch_vtable(in->prec, in->vtab[k], in->V, in->n, f.real(), f.imag(), ctx->st));
+        if ((rc = inst_alloc(in, in->n * cs + (in->fx ? cs : 0), &in->vtab[k]))) return rc;
+        if (in->fx) QSG_CUDA(cudaMemsetAsync(static_cast<char *>(in->vtab[k]) + in->n * cs, 0, cs, ctx->st));
+        QSG_CUDA(qsg::launch_vtable(tab_prec(in), in->vtab[k], in->V, in->n, f.real(), f.imag(), ctx->st));
     }
     if (in->dim == 1 && in->boundary == QSG_INFINITE_WALL && !in->wall_ext) {
         // ExpT wall: K_i = exp(f i^2), f = -i DT dt t / hbar, DT = Dp^2/(2m), Dp = hbar pi/(dx N),
@@ -1266,7 +1275,7 @@ int build_tables(qsg_inst *in)
             const cd a = in->order == 2 ? alpha : alpha * tc[k];
             if (in->prec == 0) {
                 if ((rc = inst_alloc(in, in->n * cs, &in->ktab[k]))) return rc;
-                QSG_CUDA(qsg::launch_ktable2d(in->ktab[k], in->nx, in->ny, a.real(), a.imag(), DTx, DTy,
+                QSG_CUDA(qsg::launch_ktable2d(tab_prec(in), in->ktab[k], in->nx, in->ny, a.real(), a.imag(), DTx, DTy,
                                               1.0 / ((double)in->nx * in->ny), ctx->st));
             } else {
                 const cd fx = a * DTx, fy = a * DTy;
@@ -2108,6 +2117,12 @@ int qsg_create_2d(qsg_ctx *ctx, uint64_t nx, uint64_t ny, double dx, double dy, 
     in->prec = precision;
     in->st = ctx->st;
     int rc = QSG_OK;
+    {
+        // unit-modulus factors: a real time step (and phases that stay finite)
+        const double kx = kPi / dx * hbar, ky = kPi / dy * hbar;
+        in->fx = precision == 0 && pow2_plan && dt_im == 0 &&
+                 std::isfinite((kx * kx + ky * ky) / (2 * mass) * dt_re * 2 / hbar);
+    }
     if (pow2_plan) {
         load_plans(ctx);
         auto it = ctx->plans.find(std::make_tuple(precision, (int)nx, (int)ny));

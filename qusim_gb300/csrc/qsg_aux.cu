@@ -93,12 +93,31 @@ template <> __device__ __forceinline__ float2 phase_entry<float2>(double x, doub
     return cexpm1_f(x, y);
 }
 
+// fixed-point factors (fixw, qsg_fix.cuh) of a unit-modulus phase exp(i y): the
+// double factor as hi 2^-30 + lo 2^-62
+__device__ __forceinline__ int2 fix_part(double c)
+{
+    const double s = c * 0x1p30, h = rint(s);
+    const double l = rint((s - h) * 0x1p32);
+    return make_int2((int)h, (int)fmin(fmax(l, -2147483647.0), 2147483647.0));
+}
+template <> __device__ __forceinline__ fixw phase_entry<fixw>(double, double y, double)
+{
+    const double2 r = cexp_d(0.0, y);
+    const int2 a = fix_part(r.x), b = fix_part(r.y);
+    return make_int4(a.x, a.y, b.x, b.y);
+}
+
 template <class C>
 __global__ void k_vtable(C *out, const double *V, size_t n, double fre, double fim)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double v = V[i];
         out[i] = phase_entry<C>(fre * v, fim * v, 1.0);
+        // fixed point: the flag entry (zeroed by the host) tells of a phase that is not finite
+        if constexpr (std::is_same<C, fixw>::value) {
+            if (!isfinite(fim * v)) out[n].x = 1;
+        }
     }
 }
 
@@ -134,7 +153,8 @@ __global__ void k_ktable_fs(C *out, int n1, int n2, double fre, double fim, doub
     }
 }
 
-__global__ void k_ktable2d(double2 *out, int nx, int ny, double are, double aim, double dtx, double dty,
+template <class C>
+__global__ void k_ktable2d(C *out, int nx, int ny, double are, double aim, double dtx, double dty,
                            double scale)
 {
     const size_t n = (size_t)nx * ny;
@@ -143,7 +163,7 @@ __global__ void k_ktable2d(double2 *out, int nx, int ny, double are, double aim,
         const int i = int(idx / ny), j = int(idx % ny);
         const double fi = double(i > nx / 2 ? nx - i : i), fj = double(j > ny / 2 ? ny - j : j);
         const double s = (fi * fi) * dtx + (fj * fj) * dty;
-        out[idx] = phase_entry<double2>(are * s, aim * s, scale);
+        out[idx] = phase_entry<C>(are * s, aim * s, scale);
     }
 }
 
@@ -254,6 +274,8 @@ cudaError_t launch_vtable(int prec, void *out, const double *V, size_t n, double
 {
     if (prec == 1)
         k_vtable<float2><<<blocks_for(n), kThreads, 0, st>>>((float2 *)out, V, n, fre, fim);
+    else if (prec == 3)
+        k_vtable<fixw><<<blocks_for(n), kThreads, 0, st>>>((fixw *)out, V, n, fre, fim);
     else
         k_vtable<double2><<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, V, n, fre, fim);
     return cudaGetLastError();
@@ -264,6 +286,8 @@ cudaError_t launch_ktable1d(int prec, void *out, int n, double fre, double fim, 
 {
     if (prec == 1)
         k_ktable1d<float2><<<blocks_for(n), kThreads, 0, st>>>((float2 *)out, n, fre, fim, scale);
+    else if (prec == 3)
+        k_ktable1d<fixw><<<blocks_for(n), kThreads, 0, st>>>((fixw *)out, n, fre, fim, scale);
     else
         k_ktable1d<double2><<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, n, fre, fim, scale);
     return cudaGetLastError();
@@ -301,6 +325,8 @@ cudaError_t launch_ktable_wall(int prec, void *out, int n, double fre, double fi
 {
     if (prec == 1)
         k_ktable_wall<float2><<<blocks_for(n), kThreads, 0, st>>>((float2 *)out, n, fre, fim, scale);
+    else if (prec == 3)
+        k_ktable_wall<fixw><<<blocks_for(n), kThreads, 0, st>>>((fixw *)out, n, fre, fim, scale);
     else
         k_ktable_wall<double2><<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, n, fre, fim, scale);
     return cudaGetLastError();
@@ -312,16 +338,21 @@ cudaError_t launch_ktable_fs(int prec, void *out, int n1, int n2, double fre, do
     const size_t n = (size_t)n1 * n2;
     if (prec == 1)
         k_ktable_fs<float2><<<blocks_for(n), kThreads, 0, st>>>((float2 *)out, n1, n2, fre, fim, scale);
+    else if (prec == 3)
+        k_ktable_fs<fixw><<<blocks_for(n), kThreads, 0, st>>>((fixw *)out, n1, n2, fre, fim, scale);
     else
         k_ktable_fs<double2><<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, n1, n2, fre, fim, scale);
     return cudaGetLastError();
 }
 
-cudaError_t launch_ktable2d(void *out, int nx, int ny, double are, double aim, double dtx,
+cudaError_t launch_ktable2d(int prec, void *out, int nx, int ny, double are, double aim, double dtx,
                             double dty, double scale, cudaStream_t st)
 {
-    k_ktable2d<<<blocks_for((size_t)nx * ny), kThreads, 0, st>>>((double2 *)out, nx, ny, are, aim, dtx,
-                                                                  dty, scale);
+    const unsigned blocks = blocks_for((size_t)nx * ny);
+    if (prec == 3)
+        k_ktable2d<<<blocks, kThreads, 0, st>>>((fixw *)out, nx, ny, are, aim, dtx, dty, scale);
+    else
+        k_ktable2d<<<blocks, kThreads, 0, st>>>((double2 *)out, nx, ny, are, aim, dtx, dty, scale);
     return cudaGetLastError();
 }
 

@@ -6,7 +6,12 @@
 
 namespace qsg {
 
-// out[i] = exp(f * V[i]) (fp64 tables) or exp(f * V[i]) - 1 (complex64 tables).
+// Table forms (prec): 0 the factor in double, 1 complex64 factor - 1, 3 the factor
+// in fixed point (fixw, qsg_fix.cuh; real time steps, f imaginary; `scale` is
+// left out: the passes put it into the line's exponent).
+//
+// out[i] = exp(f * V[i]) (fp64 tables; fixed point: n + 1 entries, the last the
+// flag entry, zeroed before) or exp(f * V[i]) - 1 (complex64 tables).
 // f = -i dt c / hbar: SplittingMethod2D::InitExpV (src/SplittingMethod2D.cpp:38-54).
 cudaError_t launch_vtable(int prec, void *out, const double *V, size_t n, double fre, double fim,
                           cudaStream_t st);
@@ -22,7 +27,7 @@ cudaError_t launch_ktable_fs(int prec, void *out, int n1, int n2, double fre, do
                              cudaStream_t st);
 // fp64 2D kinetic table: scale * exp(alpha (fold(i)^2 DTx + fold(j)^2 DTy)), index j + i*ny
 // (MulExpK2D on ones, src/SplittingMethod2D.cpp:56-79, src/DeviceTemplate.h:794-819).
-cudaError_t launch_ktable2d(void *out, int nx, int ny, double are, double aim, double dtx,
+cudaError_t launch_ktable2d(int prec, void *out, int nx, int ny, double are, double aim, double dtx,
                             double dty, double scale, cudaStream_t st);
 
 // psi0 (complex128) and V sampled on the device from a packet-plus-bumps

@@ -51,7 +51,7 @@ cudaError_t launch_col_kinetic(int prec, const Geom2D &g, const ColPassArgs &a, 
     if (prec == 1) {
         switch (g.m) { QSG_M_CASES(X, float) default: break; }
     } else {
-        switch (g.m) { QSG_M_CASES(X, double) default: break; }
+        switch (g.m) { QSG_M_CASES(X, double) X(double, 4096) default: break; }
     }
 #undef X
     return cudaErrorNotSupported;
@@ -96,13 +96,13 @@ bool geom2d(int prec, int nx, int ny, const Plan2D &p, Geom2D *g)
     g->m = nx / p.g;
     if (!col_variant_exists(prec, g->m, p.col_e, p.col_w)) return false;
     g->row_e = p.row_e;
-    g->row_b = tm ? 1 : row_b_for(ny, p.row_e, p.g);
+    g->row_b = tm ? 1 : row_b_for(ny, p.row_e, p.g, p.row_nt);
     g->row_threads = p.row_nt;
-    g->row_rs = tm ? p.g : row_work_for(ny, p.row_e, p.g) / p.row_nt;
+    g->row_rs = tm ? p.g : row_work_for(ny, p.row_e, p.g, p.row_nt) / p.row_nt;
     if (g->m % g->row_b) return false;
     g->row_blocks = g->m / g->row_b;
     // the TMEM pass sizes its own shared memory (one line per thread group)
-    g->row_smem = tm ? 0 : row_smem_for(csz, ny, p.row_e, p.g);
+    g->row_smem = tm ? 0 : row_smem_for(csz, ny, p.row_e, p.g, p.row_nt);
     g->col_e = p.col_e;
     g->col_w = p.col_w;
     if (ny % p.col_w) return false;
@@ -114,18 +114,20 @@ bool geom2d(int prec, int nx, int ny, const Plan2D &p, Geom2D *g)
     g->kin_threads = g->kin_w * (g->m / g->kin_e);
     g->kin_smem = (size_t)csz * col_tile_elems(csz, g->m, g->kin_w);
     const size_t smem_max = 227 * 1024 - 1024;
-    return g->row_threads <= 1024 && g->col_threads <= 512 && g->kin_threads <= 512 &&
+    // complex128 columns of 4096 only without an x split (nx = 4096)
+    const int mmax = prec == 0 && p.g == 1 ? 4096 : 2048;
+    return g->row_threads <= 1024 && g->col_threads <= (g->m == 4096 ? 1024 : 512) && g->kin_threads <= 512 &&
            g->row_smem <= smem_max && g->col_smem <= smem_max && g->kin_smem <= smem_max &&
-           g->m >= 128 && g->m <= 2048;
+           g->m >= 128 && g->m <= mmax;
 }
 
 int candidate_plans(int prec, int nx, int ny, Plan2D *out, int cap)
 {
     int n = 0;
-    const int es[2] = {16, 8};
-    const int ces[3] = {16, 8, 32};
+    const int es[3] = {16, 8, 4};
+    const int ces[4] = {16, 8, 32, 4};
     const int ws[5] = {4, 8, 16, 32, 2};
-    const int nts[3] = {512, 256, 1024};
+    const int nts[5] = {512, 256, 1024, 128, 64};
     for (int g = 1; g <= 4; g *= 2)
         for (int re : es)
             for (int nt : nts)
@@ -173,12 +175,23 @@ bool default_plan(int prec, int nx, int ny, Plan2D *p)
             c.row_kind = 1;
         }
     } else {
-        c.g = nx > 2048 ? nx / 2048 : 1;
-        c.row_e = 8;
-        c.row_nt = row_work_for(ny, 8, c.g) >= 512 ? 512 : 256;
-        c.col_e = 8;
+        // the x split's stages would run in FP64 (2 instructions per clock): only
+        // the 8192-row grids, whose columns do not fit a CTA, take one (4096^2:
+        // 714 + 595 us a column and a row pass unsplit, 570 + 860 split in two).
+        c.g = nx > 4096 ? nx / 2048 : 1;
         const int m = nx / c.g;
-        c.col_w = m >= 2048 ? 2 : (m >= 512 ? 4 : (m == 256 ? 8 : 16));
+        // Small grids are bound by the instructions one thread runs in a row: four
+        // elements a thread instead of eight (128 x 128: 10.2 against 12.4 us a
+        // pass; at 512^2 the chip is full and eight win, 15.9 + 14.5 against
+        // 18.6 + 16.2).
+        const bool small = (long)nx * ny <= 65536 && m <= 256 && ny <= 256 && c.g == 1;
+        c.row_e = small ? 4 : 8;
+        // the fewest threads that hold whole rows: more, shorter units (1024^2: 35.6
+        // with 128 threads against 41.0 us with 256)
+        const int tl = ny / c.row_e;
+        c.row_nt = c.g > 1 ? (row_work_for(ny, 8, c.g, 256) >= 512 ? 512 : 256) : small ? 128 : (tl > 64 ? tl : 64);
+        c.col_e = small ? 4 : 8;
+        c.col_w = small || m >= 1024 ? 2 : 4;
     }
     Geom2D g;
     if (geom2d(prec, nx, ny, c, &g)) {

@@ -46,14 +46,15 @@ static inline unsigned persistent_grid(K kernel, int threads, size_t smem, int u
 // Row pass: B groups of G rows per CTA so a CTA holds >= 256 threads of line
 // work; the NT threads of a CTA (256 or 512) go over its NL = B*G lines in
 // RS = NL*(NY/E)/NT rounds (NT >= NY/E: a line is never split across rounds).
-constexpr int row_b_for(int ny, int e, int g)
+// Plans of fewer threads (complex128, small grids) hold fewer groups instead.
+constexpr int row_b_for(int ny, int e, int g, int nt)
 {
-    return (256 / (g * (ny / e))) > 1 ? 256 / (g * (ny / e)) : 1;
+    return ((nt < 256 ? nt : 256) / (g * (ny / e))) > 1 ? (nt < 256 ? nt : 256) / (g * (ny / e)) : 1;
 }
-constexpr int row_work_for(int ny, int e, int g) { return row_b_for(ny, e, g) * g * (ny / e); }
-constexpr size_t row_smem_for(int csz, int ny, int e, int g)
+constexpr int row_work_for(int ny, int e, int g, int nt) { return row_b_for(ny, e, g, nt) * g * (ny / e); }
+constexpr size_t row_smem_for(int csz, int ny, int e, int g, int nt)
 {
-    return (size_t)csz * row_b_for(ny, e, g) * g * (ny + (ny >> (csz == 8 ? 4 : 3)));
+    return (size_t)csz * row_b_for(ny, e, g, nt) * g * (ny + (ny >> (csz == 8 ? 4 : 3)));
 }
 
 // Instantiated variants.  X(T, NY, E, G, NT) for the row pass (NT threads),
@@ -78,6 +79,10 @@ constexpr size_t row_smem_for(int csz, int ny, int e, int g)
     X(float, 4096, 8, 1, 512) X(float, 4096, 8, 2, 512) X(float, 4096, 8, 4, 512)
 #define QSG_ROW_VARIANTS_F64(X) \
     QSG_ROW_SMALL(X, double, 8) \
+    X(double, 128, 8, 1, 64) X(double, 128, 8, 1, 128) X(double, 256, 8, 1, 64) X(double, 256, 8, 1, 128) \
+    X(double, 512, 8, 1, 64) X(double, 512, 8, 1, 128) X(double, 1024, 8, 1, 128) \
+    X(double, 128, 4, 1, 64) X(double, 128, 4, 1, 128) X(double, 256, 4, 1, 64) X(double, 256, 4, 1, 128) \
+    X(double, 512, 4, 1, 128) X(double, 1024, 4, 1, 256) \
     X(double, 2048, 8, 1, 256) X(double, 2048, 8, 2, 512) X(double, 2048, 8, 4, 512) \
     X(double, 4096, 8, 1, 512) X(double, 4096, 8, 2, 512)
 
@@ -92,18 +97,21 @@ constexpr size_t row_smem_for(int csz, int ny, int e, int g)
     C(float, 512, 8, 4) C(float, 512, 8, 8) \
     C(float, 1024, 8, 4)
 #define QSG_COL_VARIANTS_F64(C) \
-    C(double, 128, 8, 8) C(double, 128, 8, 16) \
-    C(double, 256, 8, 4) C(double, 256, 8, 8) \
-    C(double, 512, 8, 4) \
-    C(double, 1024, 8, 4) \
-    C(double, 2048, 8, 2)
+    C(double, 128, 8, 2) C(double, 128, 8, 4) C(double, 128, 8, 8) C(double, 128, 8, 16) \
+    C(double, 256, 8, 2) C(double, 256, 8, 4) C(double, 256, 8, 8) \
+    C(double, 512, 8, 2) C(double, 512, 8, 4) \
+    C(double, 1024, 8, 2) C(double, 1024, 8, 4) \
+    C(double, 2048, 8, 2) \
+    C(double, 4096, 8, 2) \
+    C(double, 128, 4, 2) C(double, 128, 4, 4) C(double, 256, 4, 2) C(double, 256, 4, 4) \
+    C(double, 512, 4, 2) C(double, 512, 4, 4) C(double, 1024, 4, 2)
 
 // the kinetic-energy column transform: one variant per (precision, M)
 constexpr int kin_e_for(int prec) { return prec == 1 ? 16 : 8; }
 constexpr int kin_w_for(int prec, int m)
 {
     return prec == 1 ? (m >= 2048 ? 4 : (m >= 512 ? 8 : 256 / (m / 16)))
-                     : (m >= 2048 ? 2 : (m >= 512 ? 4 : 256 / (m / 8)));
+                     : (m >= 4096 ? 1 : (m >= 2048 ? 2 : (m >= 512 ? 4 : 256 / (m / 8))));
 }
 
 }  // namespace qsg

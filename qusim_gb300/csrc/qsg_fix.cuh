@@ -13,7 +13,10 @@
 // stage left, a reduction that rides on the exchange's barrier), so every
 // rounding is at most 2^-57 of the line's largest value, where a double's is
 // 2^-53 of each value.  An FFT's error is relative to the line's norm in either
-// arithmetic; measured figures stand at line_fft_fix.
+// arithmetic.  Against 80-bit runs of the same steps the error fell on every
+// shape tried (1D 64 .. 131072, Bluestein and wall lines, 2D 128^2 .. 512^2,
+// packets and white noise): 0.12 to 0.8 of the FP64 transforms' error, e.g.
+// 1.4e-14 -> 3.6e-15 after 30 O4 steps at n = 4096.
 //
 // A unit-modulus factor w is stored as {re hi, re lo, im hi, im lo}: hi =
 // round(w 2^30), lo = the rest at 2^-62, so w is held to 2^-63.
@@ -237,102 +240,180 @@ template <int E> __device__ __forceinline__ void fix_norm(Fix (&v)[E], unsigned 
     }
 }
 
-// One Stockham stage on fixed point (fft_stage's data movement); ex follows the scale.
-template <int L, int E, int S, class Lay, class Bar>
-__device__ __forceinline__ void fix_stage(Fix (&x)[E], Fix *sm, unsigned *words, const Lay &lay, const Bar &bar, int t,
-                                          const fixw *__restrict__ tw, int &ex)
-{
-    using P = Plan<L, E>;
-    constexpr int RL = P::radix_log(S);
-    constexpr int R = 1 << RL;
-    static_assert(R <= 8, "radix 2, 4 or 8: the head room above 2^61 / 4 units is 8 sqrt(2)");
-    constexpr int PL = P::p_log(S);
-    constexpr int PP = 1 << PL;
-    constexpr int J = E / R;
-    constexpr int TL = P::TL;
-    constexpr int TWO = P::tw_offset(S);
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-        Fix v[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = x[j + q * J];
-        if constexpr (PP > 1) {
-            const int k = (t + j * TL) & (PP - 1);
-            v[0].x = (v[0].x + 2) >> 2;
-            v[0].y = (v[0].y + 2) >> 2;
-#pragma unroll
-            for (int q = 1; q < R; ++q) v[q] = fix_twmul(v[q], __ldg(&tw[TWO + (q - 1) * PP + k]));
-        }
-        dft<R, false, Fix, fixw>(v);
-#pragma unroll
-        for (int q = 0; q < R; ++q) x[j + q * J] = v[q];
+// A phase table of fixed-point factors ends in a flag entry, not zero when a
+// factor was not finite (an infinite potential): such a table makes every line
+// it multiplies NaN, as the factor itself would after the next transform.
+__device__ __forceinline__ bool fix_flagged(const fixw *entry) { return __ldg(&entry->x) != 0; }
+
+// A complex128 line held in fixed point by its threads: slot e of thread t is
+// element t + e L / E, as in the register lines of qsg_fft.cuh, with value
+// v 2^ex.  Transforms and unit-modulus products chain without going back to
+// double.  Magnitudes (of the complex values, in units): a transform takes
+// |v| <= 2^59.5 and leaves |v| < 2^63 / sqrt(2); scale() brings components
+// below 2^61; a product takes that and leaves |v| <= 2^59.5.
+//
+// Reductions beyond one warp go through four words in the padding of the
+// exchange buffer: word 0 for load(), words 1 .. 3 in turn for the others.  A
+// reduction's word is zeroed before the barrier of the reduction before it,
+// when the word's last readers (three reductions back) are behind a barrier.
+template <int L, int E> struct FixLine {
+    Fix v[E];
+    int ex;
+    int r;        // next reduction's word
+    bool finite;  // false: the line holds an infinity or a NaN, and so do all its results
+
+    template <class Lay> static __device__ __forceinline__ unsigned *words(double2 *smd, const Lay &lay)
+    {
+        return reinterpret_cast<unsigned *>(smd + lay.pad_slot());
     }
-    if constexpr (PP > 1) ex += 2;
-    if constexpr (S + 1 < P::NST) {
-        using Red = FixReduce<TL, Lay, 0>;
-        constexpr int WD = 1 + (S & 1);  // this exchange's word (zeroed in the exchange before)
-        const unsigned m = Red::put(fix_or(x), words + WD);
-        bar();  // every reader of the previous stage is done with the buffer
-        if constexpr (!Red::WARP) {
-            if (lay.leader(t)) words[3 - WD] = 0;  // the next exchange's word
+    // double line -> fixed point.  x is the line (changed where it is tiny).
+    template <class Lay, class Bar>
+    __device__ __forceinline__ void load(double2 (&x)[E], double2 *smd, const Lay &lay, const Bar &bar, int t)
+    {
+        static_assert(sizeof(Fix) == sizeof(double2), "the exchange buffer is shared");
+        using Red = FixReduce<L / E, Lay, 1>;
+        unsigned *w = words(smd, lay);
+        unsigned mx = fix_absmax(x);
+        if constexpr (Red::WARP) {
+            mx = Red::put(mx, w);
+        } else {
+            // word 0's last readers are behind a later barrier; the others' may still be
+            // reading until every thread is here
+            if (lay.leader(t)) w[0] = 0;
+            bar();
+            Red::put(mx, w);
+            if (lay.leader(t)) w[1] = 0;
+            bar();
+            mx = Red::get(mx, w);
         }
+        r = 1;
+        ex = fix_in(x, v, mx, &finite);
+    }
+    __device__ __forceinline__ void store(double2 (&x)[E]) const { fix_out(v, x, ex, finite); }
+    __device__ __forceinline__ void conj()
+    {
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e].y = -v[e].y;
+    }
+    __device__ __forceinline__ static int after(int i) { return i == 3 ? 1 : i + 1; }
+
+    // components below 2^61, the largest not far below (after a transform, before a product)
+    template <class Lay, class Bar>
+    __device__ __forceinline__ void scale(double2 *smd, const Lay &lay, const Bar &bar, int t)
+    {
+        using Red = FixReduce<L / E, Lay, 0>;
+        unsigned *w = words(smd, lay);
+        const unsigned m = Red::put(fix_or(v), w + r);
+        if constexpr (!Red::WARP) {
+            if (lay.leader(t)) w[after(r)] = 0;
+            bar();
+        }
+        fix_norm(v, Red::get(m, w + r), ex);
+        if constexpr (!Red::WARP) r = after(r);
+    }
+    // v *= f(e), `twice`: two products (the reference's two multiplies by one table value)
+    template <class F> __device__ __forceinline__ void mul(F f, bool twice)
+    {
+        if (twice) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const fixw m = f(e);
+                v[e] = fix_twmul(fix_twmul(v[e], m), m);
+            }
+            ex += 4;
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[e] = fix_twmul(v[e], f(e));
+            ex += 2;
+        }
+    }
+    // the product's change of scale without a product
+    __device__ __forceinline__ void quarter()
+    {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            v[e].x = (v[e].x + 2) >> 2;
+            v[e].y = (v[e].y + 2) >> 2;
+        }
+        ex += 2;
+    }
+
+    // one Stockham stage (fft_stage's data movement)
+    template <int S, class Lay, class Bar>
+    __device__ __forceinline__ void stage(double2 *smd, const Lay &lay, const Bar &bar, int t, const fixw *__restrict__ tw)
+    {
+        using P = Plan<L, E>;
+        constexpr int RL = P::radix_log(S);
+        constexpr int R = 1 << RL;
+        static_assert(R <= 8, "radix 2, 4 or 8: a radix-8 sum grows by at most 8");
+        constexpr int PL = P::p_log(S);
+        constexpr int PP = 1 << PL;
+        constexpr int J = E / R;
+        constexpr int TL = P::TL;
+        constexpr int TWO = P::tw_offset(S);
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            const int b = t + j * TL;
-            const int k = b & (PP - 1);
-            const int o = ((b - k) << RL) + k;
+            Fix u[R];
 #pragma unroll
-            for (int q = 0; q < R; ++q) sm[lay(o + q * PP)] = x[j + q * J];
+            for (int q = 0; q < R; ++q) u[q] = v[j + q * J];
+            if constexpr (PP > 1) {
+                const int k = (t + j * TL) & (PP - 1);
+                u[0].x = (u[0].x + 2) >> 2;
+                u[0].y = (u[0].y + 2) >> 2;
+#pragma unroll
+                for (int q = 1; q < R; ++q) u[q] = fix_twmul(u[q], __ldg(&tw[TWO + (q - 1) * PP + k]));
+            }
+            dft<R, false, Fix, fixw>(u);
+#pragma unroll
+            for (int q = 0; q < R; ++q) v[j + q * J] = u[q];
         }
-        bar();
+        if constexpr (PP > 1) ex += 2;
+        if constexpr (S + 1 < P::NST) {
+            Fix *sm = reinterpret_cast<Fix *>(smd);
+            using Red = FixReduce<TL, Lay, 0>;
+            unsigned *w = words(smd, lay);
+            const unsigned m = Red::put(fix_or(v), w + r);
+            bar();  // every reader of the previous stage is done with the buffer
+            if constexpr (!Red::WARP) {
+                if (lay.leader(t)) w[after(r)] = 0;
+            }
 #pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = sm[lay(t + e * TL)];
-        fix_norm(x, Red::get(m, words + WD), ex);
+            for (int j = 0; j < J; ++j) {
+                const int b = t + j * TL;
+                const int k = b & (PP - 1);
+                const int o = ((b - k) << RL) + k;
+#pragma unroll
+                for (int q = 0; q < R; ++q) sm[lay(o + q * PP)] = v[j + q * J];
+            }
+            bar();
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[e] = sm[lay(t + e * TL)];
+            fix_norm(v, Red::get(m, w + r), ex);
+            if constexpr (!Red::WARP) r = after(r);
+        }
     }
-}
-
-template <int L, int E, int S, class Lay, class Bar>
-__device__ __forceinline__ void fix_stages(Fix (&x)[E], Fix *sm, unsigned *words, const Lay &lay, const Bar &bar, int t,
-                                           const fixw *__restrict__ tw, int &ex)
-{
-    if constexpr (S < Plan<L, E>::NST) {
-        fix_stage<L, E, S>(x, sm, words, lay, bar, t, tw, ex);
-        fix_stages<L, E, S + 1>(x, sm, words, lay, bar, t, tw, ex);
+    template <int S = 0, class Lay, class Bar>
+    __device__ __forceinline__ void fft(double2 *smd, const Lay &lay, const Bar &bar, int t, const fixw *__restrict__ tw)
+    {
+        if constexpr (S < Plan<L, E>::NST) {
+            stage<S>(smd, lay, bar, t, tw);
+            fft<S + 1>(smd, lay, bar, t, tw);
+        }
     }
-}
+};
 
 // Forward transform of a complex128 line (line_fft's contract).
 // Measured against FP64 butterflies (whole calls): 1024^2 O4 1035 -> 332 us a
 // step, a 1000-site wall 595 -> 204 us, 131072-site lines 82 -> 41 us, 450 x 700
-// 668 -> 247 us; error against 64-bit references 1.3e-14 -> 1.2e-14, 2.0e-14 ->
-// 1.3e-14, 1.2e-14 -> 1.1e-14, 8e-15 -> 4e-15 on the same runs.
+// 668 -> 247 us.
 template <int L, int E, class Lay, class Bar>
 __device__ __forceinline__ void line_fft_fix(double2 (&x)[E], double2 *smd, const Lay &lay, const Bar &bar, int t,
                                              const fixw *__restrict__ tw)
 {
-    static_assert(sizeof(Fix) == sizeof(double2), "the exchange buffer is shared");
-    static_assert(Plan<L, E>::NST >= 2, "a line has at least one exchange");
-    Fix *sm = reinterpret_cast<Fix *>(smd);
-    unsigned *words = reinterpret_cast<unsigned *>(smd + lay.pad_slot());
-    using Red = FixReduce<L / E, Lay, 1>;
-    unsigned mx = fix_absmax(x);
-    if constexpr (Red::WARP) {
-        mx = Red::put(mx, words);
-    } else {
-        // word 0's last readers are behind an exchange's barrier of the transform before; word 1
-        // (this transform's first exchange's) may still be read until every thread is here
-        if (lay.leader(t)) words[0] = 0;
-        bar();
-        Red::put(mx, words);
-        if (lay.leader(t)) words[1] = 0;
-        bar();
-        mx = Red::get(mx, words);
-    }
-    Fix v[E];
-    bool finite;
-    int ex = fix_in(x, v, mx, &finite);
-    fix_stages<L, E, 0>(v, sm, words, lay, bar, t, tw, ex);
-    fix_out(v, x, ex, finite);
+    FixLine<L, E> f;
+    f.load(x, smd, lay, bar, t);
+    f.fft(smd, lay, bar, t, tw);
+    f.store(x);
 }
 
 }  // namespace qsg

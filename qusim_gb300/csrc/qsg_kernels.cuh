@@ -72,6 +72,14 @@ __device__ __forceinline__ double2 ld_stream(const double2 *p)
     asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
     return r;
 }
+__device__ __forceinline__ fixw ld_stream(const fixw *p)
+{
+    fixw r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "l"(p));
+    return r;
+}
 template <class C> __device__ __forceinline__ void st_stream(C *p, C v) { __stcs(p, v); }
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // bulk L2 prefetch of `bytes` (a multiple of 16) from a 16-byte aligned address
@@ -145,10 +153,12 @@ __global__ void __launch_bounds__(NI *(L / E)) k_evolve1d_resident(Evolve1DBatch
 struct RowPassArgs {
     const void *in;
     void *out;
-    const void *vtab;       // V phase table (Nx*Ny), or null (plain transform)
+    const void *vtab;       // V phase table (Nx*Ny), or null (plain transform); FX: fixed-point
+                            // factors, then a flag entry (see FixFlag)
     int vtwice;             // apply it twice (the two ExpV calls at a step boundary)
     int vdiff;              // complex64: multiply by factor - 1 (the increment (V - 1) psi)
     int plain;              // complex64: tw_row / tw_nx are float2 tables (plain twiddles)
+    int fx;                 // complex128: vtab holds fixed-point factors
     const void *tw_row;     // stage-major twiddles for (Ny, E)
     const void *tw_nx;      // full circle exp(-2 pi i m / Nx), m < Nx (x-split twiddles)
     double *partials;       // per-unit sum |psi|^2 (natural-output passes), or null
@@ -173,7 +183,11 @@ struct RowPassArgs {
 template <class C, bool PL> using pass_tw_t = std::conditional_t<PL, float2, tw_t<C>>;
 template <class C, bool PL> using pass_stw_t = std::conditional_t<PL, float2, stw_t<C>>;
 
-template <class T, int NY, int E, int G, int B, int RS, bool IN, bool PL>
+// FX (complex128 with a real time step, so unit-modulus factors): a line goes
+// to fixed point once, runs transform, potential product and transform there,
+// and comes back once (1024^2, with the plans of shorter units: 53 -> 36 us a
+// row pass, 60 -> 44 us a column pass).
+template <class T, int NY, int E, int G, int B, int RS, bool IN, bool PL, bool FX>
 __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned char *smraw, double *red)
 {
     using C = cplx_t<T>;
@@ -231,6 +245,7 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
     for (int u = blockIdx.x; u < a.units; u += gridDim.x) {
     const int unext = u + gridDim.x;
     if (u != (int)blockIdx.x) cbar();  // the previous unit's readers of sm are done
+    const bool vbad = FX && vt && fix_flagged(reinterpret_cast<const fixw *>(vt) + (size_t)a.nx * NY);
     if (vt && tid < NL) {
         // each line's potential row is read right after its inverse transform:
         // start pulling the unit's rows into L2 now, one bulk prefetch per row
@@ -297,6 +312,29 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
         // [row iFFT] -> V -> [row FFT], the iFFT as conj(FFT(conj(x)))
         const int npass = (in_split ? 1 : 0) + (out_split ? 1 : 0);
         const int vpos = in_split ? 1 : 0;
+        if constexpr (FX) {
+            FixLine<NY, E> f;
+            f.load(x, sm, lay, lbar, t);
+            if (vbad) f.finite = false;
+            if (in_split) f.conj();
+#pragma unroll 1
+            for (int p = 0; p <= npass; ++p) {
+                if (p == vpos) {
+                    if (in_split) {
+                        f.conj();
+                        f.scale(sm, lay, lbar, t);
+                    }
+                    if (vt) {
+                        const fixw *vr = opaque(reinterpret_cast<const fixw *>(vt)) + (size_t)row * NY + t;
+                        f.mul([&](int e) { return ld_stream(vr + e * TL); }, a.vtwice != 0);
+                    } else {
+                        f.quarter();
+                    }
+                }
+                if (p < npass) f.fft(sm, lay, lbar, t, opaque(tw));
+            }
+            f.store(x);
+        } else {
         if (in_split) {
 #pragma unroll
             for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
@@ -334,6 +372,7 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
                 }
             }
             if (p < npass) line_fft<C, NY, E, false>(x, sm, lay, lbar, t, tw);
+        }
         }
         if (!out_split) {
             C *orow = const_cast<C *>(opaque(out)) + (size_t)row * NY + t;
@@ -392,15 +431,18 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
 // One kernel serves the three pass kinds of a step (runtime flags); the body
 // is specialised on in_split so that the registers holding the next unit's
 // input exist only where that input is split-k.
-template <class T, int NY, int E, int G, int B, int RS, bool PL = false>
-__global__ void __launch_bounds__(B *G *(NY / E) / RS) k_row_pass(RowPassArgs a)
+// complex128 runs at three CTAs of 256 threads per SM (85 registers): with two
+// (126) its integer pipes wait more (1024^2: 51.5 -> 43.3 us per launch).
+template <class T, int NY, int E, int G, int B, int RS, bool PL = false, bool FX = false>
+__global__ void __launch_bounds__(B *G *(NY / E) / RS, sizeof(T) == 8 && G == 1 ? 768 / (B * G * (NY / E) / RS) : 1)
+    k_row_pass(RowPassArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[32];
     if (a.in_split)
-        row_pass_units<T, NY, E, G, B, RS, true, PL>(a, smraw, red);
+        row_pass_units<T, NY, E, G, B, RS, true, PL, FX>(a, smraw, red);
     else
-        row_pass_units<T, NY, E, G, B, RS, false, PL>(a, smraw, red);
+        row_pass_units<T, NY, E, G, B, RS, false, PL, FX>(a, smraw, red);
 }
 
 struct ColPassArgs {
@@ -412,9 +454,11 @@ struct ColPassArgs {
     int *err;               // counter a pass whose bounded waits ran out adds 1 to (TMA pass), or null
     int no_copies;          // TMA pass, failure-path test only: issue no copies, so the first wait runs out
     int plain;              // complex64: tw_col is a float2 table (plain twiddles)
+    int fx;                 // complex128: k2d holds fixed-point factors
     const void *kx;         // complex64: x kinetic factor - 1, Nx entries
     const void *ky;         // complex64: y kinetic factor - 1, Ny entries
-    const void *k2d;        // complex128: full table Nx*Ny with 1/(Nx Ny) folded in
+    const void *k2d;        // complex128: full table Nx*Ny with 1/(Nx Ny) folded in; FX: fixed-point
+                            // factors (1/(Nx Ny), a power of two, goes to the exponent)
     const void *tw_col;     // stage-major twiddles for (M, E)
     int nx, ny, g;
     float inv_n;            // 1/(Nx Ny) (complex64 path)
@@ -427,8 +471,11 @@ struct ColPassArgs {
 // Radix-32 variants are held to 128 registers so that 512 threads (two CTAs
 // of 256) share an SM.  (Four CTAs of 128 threads, W = 4, measured slower at
 // 4096^2: 168 against 119 us.)
-template <class T, int M, int E, int W, bool PL = false>
-__global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : 1) k_col_pass(ColPassArgs a)
+// complex128 is held to 64 registers (1024 threads per SM): 1024^2 60.3 -> 52.0
+// us per launch with four columns, 2048^2 209 -> 169 us with two.
+template <class T, int M, int E, int W, bool PL = false, bool FX = false>
+__global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : sizeof(T) == 8 ? 1024 / (W * (M / E)) : 1)
+    k_col_pass(ColPassArgs a)
 {
     using C = cplx_t<T>;
     using TW = pass_stw_t<C, PL>;
@@ -483,6 +530,22 @@ __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : 1)
     }
 
     // FFT -> K -> iFFT, the iFFT as conj(FFT(conj(x)))
+    if constexpr (FX) {
+        FixLine<M, E> f;
+        f.load(x, sm, lay, bar, t);
+        f.ex -= 31 - __clz(a.nx * ny);  // 1/(Nx Ny)
+#pragma unroll 1
+        for (int p = 0; p < 2; ++p) {
+            f.fft(sm, lay, bar, t, opaque(tw));
+            if (p == 0) {
+                f.scale(sm, lay, bar, t);
+                const fixw *k2 = opaque(static_cast<const fixw *>(a.k2d)) + col;
+                f.mul([&](int e) { return ld_stream(k2 + (size_t)(a.g * (t + e * TM) + q) * ny); }, false);
+            }
+            f.conj();
+        }
+        f.store(x);
+    } else {
 #pragma unroll 1
     for (int p = inv_only ? 1 : 0; p < 2; ++p) {
         line_fft<C, M, E, false>(x, sm, lay, bar, t, tw);
@@ -526,6 +589,7 @@ __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : 1)
     }
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
+    }
 
     {
         // recomputed rather than kept live across both transforms

@@ -11,9 +11,9 @@ namespace qsg {
 template <int NY, int E, int G, int NT, bool PL>
 static cudaError_t run_row_f32a(const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
 {
-    constexpr int B = row_b_for(NY, E, G);
-    constexpr int RS = row_work_for(NY, E, G) / NT;
-    static_assert(RS * NT == row_work_for(NY, E, G), "NT must divide the CTA's line work");
+    constexpr int B = row_b_for(NY, E, G, NT);
+    constexpr int RS = row_work_for(NY, E, G, NT) / NT;
+    static_assert(RS * NT == row_work_for(NY, E, G, NT), "NT must divide the CTA's line work");
     auto k = k_row_pass<float, NY, E, G, B, RS, PL>;
     cudaError_t e = prepare_smem(k, g.row_smem);
     if (e != cudaSuccess) return e;

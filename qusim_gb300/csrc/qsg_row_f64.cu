@@ -3,13 +3,13 @@
 
 namespace qsg {
 
-template <int NY, int E, int G, int NT>
+template <int NY, int E, int G, int NT, bool FX>
 static cudaError_t run_row_f64(const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
 {
-    constexpr int B = row_b_for(NY, E, G);
-    constexpr int RS = row_work_for(NY, E, G) / NT;
-    static_assert(RS * NT == row_work_for(NY, E, G), "NT must divide the CTA's line work");
-    auto k = k_row_pass<double, NY, E, G, B, RS>;
+    constexpr int B = row_b_for(NY, E, G, NT);
+    constexpr int RS = row_work_for(NY, E, G, NT) / NT;
+    static_assert(RS * NT == row_work_for(NY, E, G, NT), "NT must divide the CTA's line work");
+    auto k = k_row_pass<double, NY, E, G, B, RS, false, FX>;
     cudaError_t e = prepare_smem(k, g.row_smem);
     if (e != cudaSuccess) return e;
     static int occ = 0;
@@ -20,7 +20,8 @@ static cudaError_t run_row_f64(const Geom2D &g, const RowPassArgs &a, cudaStream
 cudaError_t launch_row_pass_f64(const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
 {
 #define X(T, NY, E, G, NT) \
-    if (g.ny == NY && g.row_e == E && g.g == G && g.row_threads == NT) return run_row_f64<NY, E, G, NT>(g, a, st);
+    if (g.ny == NY && g.row_e == E && g.g == G && g.row_threads == NT) \
+        return a.fx ? run_row_f64<NY, E, G, NT, true>(g, a, st) : run_row_f64<NY, E, G, NT, false>(g, a, st);
     QSG_ROW_VARIANTS_F64(X)
 #undef X
     return cudaErrorNotSupported;
