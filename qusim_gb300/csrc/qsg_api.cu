@@ -103,6 +103,13 @@ struct qsg_inst {
     bool blue = false;
     int blue_m = 0;
     void *bw = nullptr, *bhs = nullptr;
+    // fixed-point forms (fx), and the exponents of the scaled tables (1D: hs, K / n; 2D: hs of
+    // the two sides, the factors along x)
+    void *bwf = nullptr, *bhsf = nullptr;
+    int bhs_exp = 0, bk_exp = 0;
+    void *bwxf = nullptr, *bhsxf = nullptr, *bwyf = nullptr, *bhsyf = nullptr;
+    int bhsx_exp = 0, bhsy_exp = 0, bkx_exp[2] = {0, 0};
+    int bfs_kexp[2] = {0, 0};  // Bluestein four-step: of the two convolution kernels
     // 1D periodic n above the one-CTA Bluestein lengths: Bluestein's convolutions
     // on the four-step passes over a buffer of n = M sites (M >= 2 n_out - 1), the
     // user's n_out sites first and zeros above; bdesc: the passes' descriptors
@@ -180,6 +187,16 @@ struct qsg_inst {
 namespace {
 
 
+int ilog2_u64(uint64_t n) { return n <= 1 ? 0 : 1 + ilog2_u64(n >> 1); }
+
+// a complex128 1D instance whose factors have unit modulus: a real time step,
+// and kinetic phases that stay finite up to the highest mode (k = pi / dx)
+bool fx_1d(int precision, double dx, double mass, double hbar, double dt_re, double dt_im)
+{
+    const double k = kPi / dx * hbar;
+    return precision == QSG_FP64 && dt_im == 0 && std::isfinite(k * k / (2 * mass) * dt_re * 2 / hbar);
+}
+
 // form of the instance's phase tables (qsg_aux.h)
 int tab_prec(const qsg_inst *in) { return in->fx ? 3 : in->prec; }
 
@@ -240,6 +257,7 @@ int fs_col(qsg_inst *in, const qsg::FsInst *desc, int ninst, bool in_k, bool out
     a.in_k = in_k ? 1 : 0;
     a.out_k = out_k ? 1 : 0;
     a.wall = 0;  // a wall extension's site 0 is zeroed once per uploaded state (step1d)
+    a.fx = in->fx ? 1 : 0;
     ProfScope ps(in->ctx, "fs_col_pass", st);
     if (maps && !in->wall_ext && in->fs_tma && qsg::fs_tma_supported(in->prec, in->fsg.n2)) {
         a.maps = maps;
@@ -286,6 +304,8 @@ int fs_row(qsg_inst *in, const qsg::FsInst *desc, int ninst, int ksel, cudaStrea
     a.tw_row = in->tw_fs_row;
     a.ksel = ksel;
     a.inv_n = (float)(1.0 / (double)in->n);
+    a.fx = in->fx ? 1 : 0;
+    a.kexp[0] = a.kexp[1] = -ilog2_u64(in->n);  // 1/N
     ProfScope ps(in->ctx, "fs_row_pass", st);
     QSG_CUDA(qsg::launch_fs_row(in->prec, in->fsg, a, ninst, st));
     return QSG_OK;
@@ -330,6 +350,9 @@ int step_bfs(qsg_inst *in, uint64_t nsteps, cudaStream_t st)
         a.tw_row = in->tw_fs_row;
         a.ksel = ksel;
         a.plain = 1;
+        a.fx = in->fx ? 1 : 0;
+        a.kexp[0] = in->bfs_kexp[0];
+        a.kexp[1] = in->bfs_kexp[1];
         ProfScope ps(in->ctx, "fs_row_pass", st);
         QSG_CUDA(qsg::launch_fs_row(in->prec, in->fsg, a, 1, st));
         return QSG_OK;
@@ -370,8 +393,11 @@ int step1d(qsg_inst *in, uint64_t nsteps, int renorm)
         qsg::BlueArgs a{};
         a.psi = in->psi;
         a.tw = in->tw;
-        a.w = in->bw;
-        a.hs = in->bhs;
+        a.w = in->fx ? in->bwf : in->bw;
+        a.hs = in->fx ? in->bhsf : in->bhs;
+        a.fx = in->fx ? 1 : 0;
+        a.hs_exp = in->bhs_exp;
+        a.k_exp = in->bk_exp;
         a.vtab[0] = in->vtab[0];
         a.vtab[1] = in->vtab[1];
         a.ktab[0] = in->ktab[0];
@@ -402,6 +428,7 @@ int step1d(qsg_inst *in, uint64_t nsteps, int renorm)
         a.order = in->order;
         a.renormalize = renorm;
         a.count = 1;
+        a.fx = in->fx ? 1 : 0;
         if (in->boundary == QSG_INFINITE_WALL) {
             ProfScope ps(ctx, "evolve1d_wall", in->st);
             QSG_CUDA(qsg::launch_wall1d(in->prec, (int)in->n, a, in->st));
@@ -572,8 +599,10 @@ int step2d_blue(qsg_inst *in, uint64_t nsteps, int renorm)
         a.in_k = in_k ? 1 : 0;
         a.out_k = out_k ? 1 : 0;
         a.tw = in->btwy;
-        a.w = in->bwy;
-        a.hs = in->bhsy;
+        a.w = in->fx ? in->bwyf : in->bwy;
+        a.hs = in->fx ? in->bhsyf : in->bhsy;
+        a.fx = in->fx ? 1 : 0;
+        a.hs_exp = in->bhsy_exp;
         a.nx = in->nx;
         a.ny = in->ny;
         ProfScope ps(ctx, "row_pass_blue", in->st);
@@ -584,8 +613,11 @@ int step2d_blue(qsg_inst *in, uint64_t nsteps, int renorm)
         qsg::Blue2DArgs a{};
         a.psi = in->psi;
         a.tw = in->btwx;
-        a.w = in->bwx;
-        a.hs = in->bhsx;
+        a.w = in->fx ? in->bwxf : in->bwx;
+        a.hs = in->fx ? in->bhsxf : in->bhsx;
+        a.fx = in->fx ? 1 : 0;
+        a.hs_exp = in->bhsx_exp;
+        a.k_exp = in->bkx_exp[d];
         a.kx = in->bkx[d];
         a.ky = in->bky[d];
         a.nx = in->nx;
@@ -874,6 +906,35 @@ int upload_factors(qsg_inst *in, const std::vector<std::complex<long double>> &s
     return QSG_OK;
 }
 
+// the same as a table of fixed-point factors: src = table 2^*exp2 with the
+// table's largest modulus between 1/2 and 1, or src itself (moduli up to 1)
+// without exp2
+int upload_fixed(qsg_inst *in, const std::vector<std::complex<long double>> &src, void **dst, int *exp2)
+{
+    double m = 0;
+    if (exp2)
+        for (const auto &z : src) {
+            const double re = (double)z.real(), im = (double)z.imag();
+            m = std::max(m, std::sqrt(re * re + im * im));
+        }
+    int e = 0;
+    if (m > 0) std::frexp(m, &e);
+    const double sc = std::ldexp(1.0, -e);  // (exact: the two parts of a value scale as they are)
+    std::vector<int32_t> h(src.size() * 4);
+    auto put = [&](long double v, int32_t *q) {
+        const double v1 = (double)v, v2 = (double)(v - (long double)v1);
+        put_fixed(v1 * sc, v2 * sc, q, q + 1);
+    };
+    for (size_t i = 0; i < src.size(); ++i) {
+        put(src[i].real(), &h[4 * i]);
+        put(src[i].imag(), &h[4 * i + 2]);
+    }
+    if (int r = inst_alloc(in, h.size() * 4, dst)) return r;
+    QSG_CUDA(cudaMemcpyAsync(*dst, h.data(), h.size() * 4, cudaMemcpyHostToDevice, in->ctx->st));
+    if (exp2) *exp2 = e;
+    return QSG_OK;
+}
+
 // --- 1D plans ----------------------------------------------------------------
 
 // The timing resources of a tuner, given back on every path out: its two
@@ -999,8 +1060,8 @@ int build_ktab_1d(qsg_inst *in)
         // shared by every instance of the context with the same size and coefficient (a batch of
         // equal-dx, equal-dt instances reads one table per size from L2 instead of one each);
         // key (precision, n1, n2) for the four-step layout, (precision, n, 0) for the natural one
-        const auto key = in->fourstep ? std::make_tuple(in->prec, in->fsg.n1, in->fsg.n2, f.real(), f.imag())
-                                      : std::make_tuple(in->prec, (int)in->n, 0, f.real(), f.imag());
+        const auto key = in->fourstep ? std::make_tuple(tab_prec(in), in->fsg.n1, in->fsg.n2, f.real(), f.imag())
+                                      : std::make_tuple(tab_prec(in), (int)in->n, 0, f.real(), f.imag());
         auto it = ctx->fs_ktabs.find(key);
         const bool fresh = it == ctx->fs_ktabs.end();
         if (fresh) {
@@ -1014,10 +1075,10 @@ int build_ktab_1d(qsg_inst *in)
         in->shared_k.push_back(key);
         in->ktab[k] = it->second.p;
         if (fresh && in->fourstep) {
-            QSG_CUDA(qsg::launch_ktable_fs(in->prec, it->second.p, in->fsg.n1, in->fsg.n2, f.real(), f.imag(),
+            QSG_CUDA(qsg::launch_ktable_fs(tab_prec(in), it->second.p, in->fsg.n1, in->fsg.n2, f.real(), f.imag(),
                                            1.0 / (double)in->n, ctx->st));
         } else if (fresh) {
-            QSG_CUDA(qsg::launch_ktable1d(in->prec, it->second.p, (int)in->n, f.real(), f.imag(),
+            QSG_CUDA(qsg::launch_ktable1d(tab_prec(in), it->second.p, (int)in->n, f.real(), f.imag(),
                                           1.0 / (double)in->n, ctx->st));
         }
     }
@@ -1060,9 +1121,18 @@ int build_bfs_tables(qsg_inst *in)
     const cl mi_dt_h = cl(0, -1) * in->dt / in->hbar;
     auto phase = [&](double a, double x) { return std::exp(mi_dt_h * (a * x)); };
     // upload M natural values: complex64 as factor - 1, complex128 plain
-    auto put = [&](const std::vector<cl> &v, void **dst, bool minus_one) -> int {
-        if (int r = inst_alloc(in, M * cs, dst)) return r;
+    // (fixed point: with the flag entry; kernels scaled by 2^-*exp2)
+    auto put = [&](const std::vector<cl> &v, void **dst, bool minus_one, int *exp2 = nullptr) -> int {
+        if (int r = inst_alloc(in, M * cs + (in->fx ? cs : 0), dst)) return r;
         std::vector<unsigned char> h(M * cs);
+        int e = 0;
+        if (in->fx && exp2) {
+            double m = 0;
+            for (uint64_t i = 0; i < M; ++i)
+                m = std::max(m, v[i].real() * v[i].real() + v[i].imag() * v[i].imag());
+            if (m > 0) std::frexp(std::sqrt(m), &e);
+            *exp2 = e;
+        }
         for (uint64_t i = 0; i < M; ++i) {
             const cl z = (minus_one && in->prec == 1) ? v[i] - 1.0 : v[i];
             if (in->prec == 0) {
@@ -1074,6 +1144,7 @@ int build_bfs_tables(qsg_inst *in)
             }
         }
         QSG_CUDA(cudaMemcpyAsync(*dst, h.data(), h.size(), cudaMemcpyHostToDevice, in->ctx->st));
+        if (in->fx) QSG_CUDA(qsg::launch_fix_table(*dst, M, std::ldexp(1.0, -e), in->ctx->st));
         QSG_CUDA(cudaStreamSynchronize(in->ctx->st));  // h is pageable and goes out of scope
         return QSG_OK;
     };
@@ -1117,14 +1188,14 @@ int build_bfs_tables(qsg_inst *in)
     const uint64_t n1 = (uint64_t)in->fsg.n1, n2 = (uint64_t)in->fsg.n2;
     for (uint64_t k2 = 0; k2 < n2; ++k2)
         for (uint64_t k1 = 0; k1 < n1; ++k1) t[k2 * n1 + k1] = hs[k2 + n2 * k1];
-    if ((rc = put(t, &h1, false))) return rc;
+    if ((rc = put(t, &h1, false, &in->bfs_kexp[0]))) return rc;
     // FFT_M(h*)_k = conj(FFT_M(h)_{-k}), with the 1/n of the inverse DFT
     for (uint64_t k2 = 0; k2 < n2; ++k2)
         for (uint64_t k1 = 0; k1 < n1; ++k1) {
             const uint64_t k = k2 + n2 * k1;
             t[k2 * n1 + k1] = std::conj(hs[(M - k) % M]) / (double)n;
         }
-    if ((rc = put(t, &h2, false))) return rc;
+    if ((rc = put(t, &h2, false, &in->bfs_kexp[1]))) return rc;
     // KinEn weights of the n frequencies: fold(k)^2 DT with the periodic branch's DT
     // (it omits hbar^2, src/SplittingMethod1D.cpp:101-102), the wall's with it (:117-119;
     // |F|^2 of the odd extension is even, so the ratio over the 2n frequencies is the
@@ -1192,7 +1263,7 @@ int build_tables(qsg_inst *in)
         for (int k = 0; k < ntab; ++k) {
             const cd f = -I * DT * in->dt * tc[k] / in->hbar;
             if ((rc = inst_alloc(in, in->n * cs, &in->ktab[k]))) return rc;
-            QSG_CUDA(qsg::launch_ktable_wall(in->prec, in->ktab[k], (int)in->n, f.real(), f.imag(),
+            QSG_CUDA(qsg::launch_ktable_wall(tab_prec(in), in->ktab[k], (int)in->n, f.real(), f.imag(),
                                              -1.0 / (2.0 * (double)in->n), ctx->st));
         }
     } else if (in->dim == 1 && in->blue) {
@@ -1209,15 +1280,28 @@ int build_tables(qsg_inst *in)
             // exp(f q), f = -i DT dt t / hbar: real part DT q t Im(dt) / hbar, imaginary -DT q t Re(dt) / hbar
             for (uint64_t i = 0; i < n; ++i) {
                 const long double fo = (long double)(i > n / 2 ? n - i : i), q = fo * fo;
-                const long double re = DT * q * tc[k] * (long double)in->dt.imag() / in->hbar;
                 const long double im = -DT * q * tc[k] * (long double)in->dt.real() / in->hbar;
-                kt[k][i] = std::exp(re) * std::complex<long double>(cosl(im), sinl(im)) / (long double)n;
+                kt[k][i] = std::complex<long double>(cosl(im), sinl(im)) / (long double)n;
+                if (in->dt.imag() != 0)
+                    kt[k][i] *= std::exp(DT * q * tc[k] * (long double)in->dt.imag() / in->hbar);
             }
         }
         if ((rc = upload_factors(in, w, &in->bw))) return rc;
         if ((rc = upload_factors(in, hs, &in->bhs))) return rc;
-        for (int k = 0; k < ntab; ++k)
-            if ((rc = upload_factors(in, kt[k], &in->ktab[k]))) return rc;
+        if (in->fx) {
+            int we = 0;
+            if ((rc = upload_fixed(in, w, &in->bwf, nullptr))) return rc;
+            if ((rc = upload_fixed(in, hs, &in->bhsf, &in->bhs_exp))) return rc;
+            // (K_0 = 1 in both: one scale)
+            for (int k = 0; k < ntab; ++k) {
+                if ((rc = upload_fixed(in, kt[k], &in->ktab[k], &we))) return rc;
+                if (k > 0 && we != in->bk_exp) return fail(QSG_ERR_STATE, "Bluestein kinetic tables of different scale");
+                in->bk_exp = we;
+            }
+        } else {
+            for (int k = 0; k < ntab; ++k)
+                if ((rc = upload_factors(in, kt[k], &in->ktab[k]))) return rc;
+        }
     } else if (in->dim == 2 && in->blue2) {
         // per side: Bluestein tables; per kinetic coefficient d: exp(a d DTx fold(i)^2) / (nx ny)
         // and exp(a d DTy fold(j)^2), a = -i dt / hbar (SplittingMethod2D::InitExpT,
@@ -1226,9 +1310,15 @@ int build_tables(qsg_inst *in)
         qsg::blue_tables(in->nx, in->bmx, w, hs);
         if ((rc = upload_factors(in, w, &in->bwx))) return rc;
         if ((rc = upload_factors(in, hs, &in->bhsx))) return rc;
+        if (in->fx && ((rc = upload_fixed(in, w, &in->bwxf, nullptr)) ||
+                       (rc = upload_fixed(in, hs, &in->bhsxf, &in->bhsx_exp))))
+            return rc;
         qsg::blue_tables(in->ny, in->bmy, w, hs);
         if ((rc = upload_factors(in, w, &in->bwy))) return rc;
         if ((rc = upload_factors(in, hs, &in->bhsy))) return rc;
+        if (in->fx && ((rc = upload_fixed(in, w, &in->bwyf, nullptr)) ||
+                       (rc = upload_fixed(in, hs, &in->bhsyf, &in->bhsy_exp))))
+            return rc;
         const long double nn = (long double)in->nx * in->ny;
         for (int k = 0; k < ntab; ++k) {
             const long double d = in->order == 2 ? 1.0L : (long double)tc[k];
@@ -1240,11 +1330,13 @@ int build_tables(qsg_inst *in)
                 std::vector<std::complex<long double>> f(L);
                 for (int i = 0; i < L; ++i) {
                     const long double fo = (long double)(i > L / 2 ? L - i : i), q = fo * fo * DT * d;
-                    const long double re = q * (long double)in->dt.imag() / in->hbar;
                     const long double im = -q * (long double)in->dt.real() / in->hbar;
-                    f[i] = std::exp(re) * std::complex<long double>(cosl(im), sinl(im)) / (ax == 0 ? nn : 1.0L);
+                    f[i] = std::complex<long double>(cosl(im), sinl(im)) / (ax == 0 ? nn : 1.0L);
+                    if (in->dt.imag() != 0) f[i] *= std::exp(q * (long double)in->dt.imag() / in->hbar);
                 }
-                if ((rc = upload_factors(in, f, ax == 0 ? &in->bkx[k] : &in->bky[k]))) return rc;
+                void **dst = ax == 0 ? &in->bkx[k] : &in->bky[k];
+                rc = in->fx ? upload_fixed(in, f, dst, ax == 0 ? &in->bkx_exp[k] : nullptr) : upload_factors(in, f, dst);
+                if (rc) return rc;
             }
         }
     } else if (in->dim == 1) {
@@ -1522,7 +1614,7 @@ int apply_plan_1d(qsg_inst *in, const qsg_plan1d &p)
     if (fs) {
         if ((rc = get_twiddles(ctx, in->prec, g.n2, g.col_e, &tfc))) return rc;
         if ((rc = get_twiddles(ctx, in->prec, g.n1, g.row_e, &tfr))) return rc;
-        if ((rc = get_fs_grid(ctx, in->prec, g.n1, g.n2, &tn))) return rc;
+        if ((rc = get_fs_grid(ctx, tab_prec(in), g.n1, g.n2, &tn))) return rc;
         if ((rc = get_twiddles(ctx, in->prec, g.n1, qsg::elems_per_thread(in->prec), &tw))) return rc;
     } else {
         if ((rc = get_twiddles(ctx, in->prec, (int)in->n, qsg::elems_per_thread(in->prec), &tw))) return rc;
@@ -1863,6 +1955,7 @@ static int create_1d_locked(qsg_ctx *ctx, uint64_t n, double dx, double mass, do
     in->fs_tma = plan.tma != 0;
     in->blue = blue_m > 0;
     in->blue_m = blue_m;
+    in->fx = fx_1d(precision, dx, mass, hbar, dt_re, dt_im);
     int rc = QSG_OK;
     if (in->blue) {
         rc = get_twiddles(ctx, precision, blue_m, qsg::blue_elems(precision), &in->tw);
@@ -1872,7 +1965,7 @@ static int create_1d_locked(qsg_ctx *ctx, uint64_t n, double dx, double mass, do
     } else {
         rc = get_twiddles(ctx, precision, fsg.n2, fsg.col_e, &in->tw_fs_col);
         if (!rc) rc = get_twiddles(ctx, precision, fsg.n1, fsg.row_e, &in->tw_fs_row);
-        if (!rc) rc = get_fs_grid(ctx, precision, fsg.n1, fsg.n2, &in->tw_n);
+        if (!rc) rc = get_fs_grid(ctx, tab_prec(in), fsg.n1, fsg.n2, &in->tw_n);
         if (!rc) rc = get_twiddles(ctx, precision, (int)fsg.n1, qsg::elems_per_thread(precision), &in->tw);
     }
     if (!rc && wall_ext) {
@@ -2120,7 +2213,7 @@ int qsg_create_2d(qsg_ctx *ctx, uint64_t nx, uint64_t ny, double dx, double dy, 
     {
         // unit-modulus factors: a real time step (and phases that stay finite)
         const double kx = kPi / dx * hbar, ky = kPi / dy * hbar;
-        in->fx = precision == 0 && pow2_plan && dt_im == 0 &&
+        in->fx = precision == 0 && dt_im == 0 &&
                  std::isfinite((kx * kx + ky * ky) / (2 * mass) * dt_re * 2 / hbar);
     }
     if (pow2_plan) {
@@ -2390,12 +2483,15 @@ int qsg_energies(qsg_inst *in, double *kin, double *pot)
                 ca.vsel = 0;
                 ca.in_k = 0;
                 ca.out_k = 1;
+                ca.fx = in->fx ? 1 : 0;
                 QSG_CUDA(qsg::launch_fs_col(in->prec, in->fsg, ca, 1, ctx->st));
                 qsg::FsRowArgs ra{};
                 ra.inst = dd;
                 ra.tw_row = in->tw_fs_row;
                 ra.ksel = 0;
                 ra.plain = 1;
+                ra.fx = ca.fx;
+                ra.kexp[0] = in->bfs_kexp[0];
                 QSG_CUDA(qsg::launch_fs_row(in->prec, in->fsg, ra, 1, ctx->st));
                 ca.vsel = 1;  // no table: the descriptor's second V entry is null
                 ca.in_k = 1;
@@ -2432,6 +2528,7 @@ int qsg_energies(qsg_inst *in, double *kin, double *pot)
                 ca.vsel = 0;
                 ca.in_k = 0;
                 ca.out_k = 1;
+                ca.fx = in->fx ? 1 : 0;
                 ca.wall = in->wall_ext ? 1 : 0;  // the wall KinEn transforms psi with sites 0 and n zeroed
                 QSG_CUDA(qsg::launch_fs_col(in->prec, in->fsg, ca, 1, ctx->st));
                 qsg::FsRowArgs ra{};
@@ -2941,7 +3038,8 @@ int qsg_batch_create_1d(qsg_ctx *ctx, int count, const uint64_t *n, const double
     QSG_CUDA(cudaSetDevice(ctx->dev));
     qsg_batch *b = new qsg_batch();
     b->ctx = ctx;
-    std::map<uint64_t, int> cls;
+    // classes: members of one length and one table form (a launch runs one kernel)
+    std::map<std::pair<uint64_t, bool>, int> cls;
     for (int i = 0; i < count; ++i) {
         qsg_inst *in = nullptr;
         int rc = create_1d_locked(ctx, n[i], dx[i], mass, hbar, dt_re[i], dt_im ? dt_im[i] : 0.0, order, precision,
@@ -2958,12 +3056,12 @@ int qsg_batch_create_1d(qsg_ctx *ctx, int count, const uint64_t *n, const double
         in->batch_member = true;
         b->insts.push_back(in);
         b->sites += n[i];
-        auto it = cls.find(n[i]);
+        const auto key = std::make_pair(n[i], in->fx);
+        auto it = cls.find(key);
         if (it == cls.end()) {
-            cls[n[i]] = (int)b->classes.size();
+            it = cls.emplace(key, (int)b->classes.size()).first;
             b->classes.emplace_back();
             b->classes.back().n = n[i];
-            it = cls.find(n[i]);
         }
         b->classes[it->second].members.push_back(i);
     }
@@ -3068,6 +3166,7 @@ int batch_enqueue(qsg_batch *b, uint64_t nsteps)
             a.nsteps = nsteps;
             a.order = proto->order;
             a.count = (int)c.members.size();
+            a.fx = proto->fx ? 1 : 0;
             ProfScope ps(ctx, "evolve1d_resident", c.st);
             cudaError_t e = qsg::launch_evolve1d(proto->prec, (int)proto->n, a, c.st);
             if (e != cudaSuccess) {
@@ -3260,13 +3359,16 @@ int qsg_batch_set_plan_1d(qsg_batch *b, uint64_t n, const qsg_plan1d *p)
     if (b->broken) return fail(QSG_ERR_STATE, "qsg_batch_set_plan_1d: a failed plan switch left the batch unusable");
     std::lock_guard<std::mutex> lk(b->ctx->mu);
     QSG_CUDA(cudaSetDevice(b->ctx->dev));
-    qsg_batch::Class *c = batch_class(b, n);
-    if (!c) return fail(QSG_ERR_ARG, "qsg_batch_set_plan_1d: no member of length " + std::to_string(n));
-    qsg_inst *proto = b->insts[c->members[0]];
-    if (same_plan1d(*p, proto->plan1d)) return QSG_OK;
-    if (!plan1d_valid(proto->prec, n, QSG_PERIOD, *p))
-        return fail(QSG_ERR_UNSUPPORTED, "qsg_batch_set_plan_1d: plan not available for length " + std::to_string(n));
-    return batch_class_plan(b, *c, *p);
+    if (!batch_class(b, n)) return fail(QSG_ERR_ARG, "qsg_batch_set_plan_1d: no member of length " + std::to_string(n));
+    for (auto &c : b->classes) {
+        if (c.n != n) continue;
+        qsg_inst *proto = b->insts[c.members[0]];
+        if (same_plan1d(*p, proto->plan1d)) continue;
+        if (!plan1d_valid(proto->prec, n, QSG_PERIOD, *p))
+            return fail(QSG_ERR_UNSUPPORTED, "qsg_batch_set_plan_1d: plan not available for length " + std::to_string(n));
+        if (int rc = batch_class_plan(b, c, *p)) return rc;
+    }
+    return QSG_OK;
 }
 
 int qsg_batch_autotune(qsg_batch *b, int trial_steps, double *ms_per_step)
@@ -3290,6 +3392,13 @@ int qsg_batch_autotune(qsg_batch *b, int trial_steps, double *ms_per_step)
     for (auto &c : b->classes) {
         qsg_inst *proto = b->insts[c.members[0]];
         if (!proto->fourstep) continue;
+        if (qsg_batch::Class *tuned = batch_class(b, c.n); tuned != &c) {
+            // a length's plan is one for all its members: the first class's choice
+            const qsg_plan1d p = b->insts[tuned->members[0]]->plan1d;
+            if (!same_plan1d(p, proto->plan1d))
+                if (int rc = batch_class_plan(b, c, p)) return rc;
+            continue;
+        }
         std::vector<qsg_plan1d> cands;
         plans_1d(proto->prec, c.n, QSG_PERIOD, cands);
         cands.erase(std::remove_if(cands.begin(), cands.end(), [](const qsg_plan1d &q) { return q.kind != 1; }),
@@ -3638,11 +3747,11 @@ void srv_loop(qsg_server *S)
             ++i;
         }
         // dispatch: batched resident groups
-        std::map<std::tuple<uint64_t, int, int>, std::vector<SrvRequest *>> groups;
+        std::map<std::tuple<uint64_t, int, int, bool>, std::vector<SrvRequest *>> groups;
         for (auto &q : running)
             if (!q->in_flight && !q->fail_rc && q->dispatched < q->req.nsteps && q->req.dim == 1 &&
                 !q->inst->fourstep && !q->inst->blue)
-                groups[std::make_tuple(q->req.nx, q->req.order, q->req.precision)].push_back(q.get());
+                groups[std::make_tuple(q->req.nx, q->req.order, q->req.precision, q->inst->fx)].push_back(q.get());
         for (auto &kv : groups) {
             auto &g = kv.second;
             uint64_t chunk = 1024;
@@ -3692,6 +3801,7 @@ void srv_loop(qsg_server *S)
                 a.nsteps = chunk;
                 a.order = g[0]->req.order;
                 a.count = cnt;
+                a.fx = g[0]->inst->fx ? 1 : 0;
                 e = qsg::launch_evolve1d(g[0]->req.precision, (int)g[0]->req.nx, a, st);
                 what = "resident 1D launch";
             }

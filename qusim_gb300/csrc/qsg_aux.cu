@@ -94,18 +94,30 @@ template <> __device__ __forceinline__ float2 phase_entry<float2>(double x, doub
 }
 
 // fixed-point factors (fixw, qsg_fix.cuh) of a unit-modulus phase exp(i y): the
-// double factor as hi 2^-30 + lo 2^-62
+// double factor, |c| <= 1, as hi 2^-30 + lo 2^-62.  Its significand is shifted to
+// units of 2^-62 (in integers: FP64 roundings cost a tenth of the table build).
 __device__ __forceinline__ int2 fix_part(double c)
 {
-    const double s = c * 0x1p30, h = rint(s);
-    const double l = rint((s - h) * 0x1p32);
-    return make_int2((int)h, (int)fmin(fmax(l, -2147483647.0), 2147483647.0));
+    const long long v = fix_from(c, 1023, 10);
+    const int l = fix_lo(v);
+    return make_int2(fix_hir(v), l == (int)0x80000000 ? l + 1 : l);
 }
-template <> __device__ __forceinline__ fixw phase_entry<fixw>(double, double y, double)
+template <> __device__ __forceinline__ fixw phase_entry<fixw>(double, double y, double scale)
 {
     const double2 r = cexp_d(0.0, y);
-    const int2 a = fix_part(r.x), b = fix_part(r.y);
+    const double sg = scale < 0 ? -1.0 : 1.0;
+    const int2 a = fix_part(sg * r.x), b = fix_part(sg * r.y);
     return make_int4(a.x, a.y, b.x, b.y);
+}
+
+__global__ void k_fix_table(fixw *tab, size_t n, double scale)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const double2 z = reinterpret_cast<const double2 *>(tab)[i];
+        const int2 a = fix_part(z.x * scale), b = fix_part(z.y * scale);
+        tab[i] = make_int4(a.x, a.y, b.x, b.y);
+        if (!isfinite(z.x) || !isfinite(z.y)) tab[n].x = 1;
+    }
 }
 
 template <class C>
@@ -278,6 +290,15 @@ cudaError_t launch_vtable(int prec, void *out, const double *V, size_t n, double
         k_vtable<fixw><<<blocks_for(n), kThreads, 0, st>>>((fixw *)out, V, n, fre, fim);
     else
         k_vtable<double2><<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, V, n, fre, fim);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fix_table(void *tab, size_t n, double scale, cudaStream_t st)
+{
+    fixw *t = static_cast<fixw *>(tab);
+    const cudaError_t e = cudaMemsetAsync(t + n, 0, sizeof(fixw), st);
+    if (e != cudaSuccess) return e;
+    k_fix_table<<<blocks_for(n), kThreads, 0, st>>>(t, n, scale);
     return cudaGetLastError();
 }
 

@@ -7,8 +7,8 @@
 namespace qsg {
 
 // Table forms (prec): 0 the factor in double, 1 complex64 factor - 1, 3 the factor
-// in fixed point (fixw, qsg_fix.cuh; real time steps, f imaginary; `scale` is
-// left out: the passes put it into the line's exponent).
+// in fixed point (fixw, qsg_fix.cuh; real time steps, f imaginary; of `scale`
+// only the sign: its size goes into the line's exponent in the passes).
 //
 // out[i] = exp(f * V[i]) (fp64 tables; fixed point: n + 1 entries, the last the
 // flag entry, zeroed before) or exp(f * V[i]) - 1 (complex64 tables).
@@ -29,6 +29,9 @@ cudaError_t launch_ktable_fs(int prec, void *out, int n1, int n2, double fre, do
 // (MulExpK2D on ones, src/SplittingMethod2D.cpp:56-79, src/DeviceTemplate.h:794-819).
 cudaError_t launch_ktable2d(int prec, void *out, int nx, int ny, double are, double aim, double dtx,
                             double dty, double scale, cudaStream_t st);
+
+// n factors in double, in place, to fixed point (times scale), and the flag entry behind them
+cudaError_t launch_fix_table(void *tab, size_t n, double scale, cudaStream_t st);
 
 // psi0 (complex128) and V sampled on the device from a packet-plus-bumps
 // formula (qsg_spec), point (i, j) at x0 + i*dx, y0 + j*dy, index j + i*ny

@@ -15,13 +15,16 @@ namespace {
 
 constexpr int blue_e(int prec) { return prec == 1 ? 16 : 8; }
 
-template <class T, int M>
+template <class T, int M, bool FX = false>
 cudaError_t run_blue(const BlueArgs &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_blue<T, M, true>(a, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M);
-    auto k = k_evolve1d_blue<T, M, E>;
+    auto k = k_evolve1d_blue<T, M, E, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<1, M / E, smem, st>>>(a);
@@ -273,14 +276,17 @@ int blue_cols_per_cta(int prec, int m) { return std::max(1, std::min(16, 65536 /
 
 namespace {
 
-template <class T, int M>
+template <class T, int M, bool FX = false>
 cudaError_t run_row_blue(const Blue2DArgs &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_row_blue<T, M, true>(a, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     constexpr int RPC = (256 / (M / E)) > 1 ? 256 / (M / E) : 1;
     const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M) * RPC;
-    auto k = k_row_blue<T, M, E, RPC>;
+    auto k = k_row_blue<T, M, E, RPC, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<(a.nx + RPC - 1) / RPC, RPC * (M / E), smem, st>>>(a);
@@ -305,6 +311,11 @@ cudaError_t run_col_blue(const Blue2DArgs &a, bool kinetic, double dtx, double d
         cudaError_t e = prepare_smem(k, smem);
         if (e != cudaSuccess) return e;
         k<<<grid, W * (M / E), smem, st>>>(a, dtx, dty, partials);
+    } else if (sizeof(T) == 8 && a.fx) {
+        auto k = k_col_blue<T, M, E, W, sizeof(T) == 8>;
+        cudaError_t e = prepare_smem(k, smem);
+        if (e != cudaSuccess) return e;
+        k<<<grid, W * (M / E), smem, st>>>(a);
     } else {
         auto k = k_col_blue<T, M, E, W>;
         cudaError_t e = prepare_smem(k, smem);

@@ -47,10 +47,16 @@ struct BlueArgs {
                             // steps keep the extension as it evolves (odd to rounding; the host
                             // zeroes the caller's site 0 once per uploaded state)
     int norm_n;             // sites the norm sums (the wall's n), 0: all n
+    // complex128, real time steps: fixed-point tables (fixw) in their place; the values of hs
+    // and K / n are the tables' times 2^hs_exp and 2^k_exp
+    int fx, hs_exp, k_exp;
 };
 
-// 1D resident evolution of one instance of any length n (2n - 1 <= M)
-template <class T, int M, int E>
+// 1D resident evolution of one instance of any length n (2n - 1 <= M).
+// FX (complex128, real time steps): the line stays in fixed point for all steps,
+// and the closing chirp w* of a kinetic substep cancels against the opening w of
+// the next around the V product, which then only has to zero the slots from n on.
+template <class T, int M, int E, bool FX = false>
 __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
 {
     using C = cplx_t<T>;
@@ -113,6 +119,48 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
         for (int e = 0; e < E; ++e) x[e] = cmulc(x[e], ld_c(w + t + e * TL));
     };
     const int nsub = a.order == 2 ? 1 : 3;
+    if constexpr (FX) {
+        auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
+        auto upto_n = [&](const fixw *p) {
+            return [=](int e) { return t + e * TL < n ? __ldg(p + e * TL) : fixw{0, 0, 0, 0}; };
+        };
+        FixLine<M, E> f;
+        f.load(x, sm, lay, bar, t);
+        if (fix_flagged(tab(v0) - t + n) || (a.order == 4 && fix_flagged(tab(v1) - t + n))) f.finite = false;
+        f.mul(upto_n(tab(v0)), false);
+        f.mul([&](int e) { return __ldg(tab(w) + e * TL); }, false);
+#pragma unroll 1
+        for (uint64_t s = 0; s < a.nsteps; ++s) {
+#pragma unroll 1
+            for (int h = 0; h < 4 * nsub; ++h) {
+                // substep u of the step: x -> FFT -> conj(. hs) -> FFT -> . conj(K / n) -> FFT ->
+                // conj(. hs) -> FFT -> V
+                const int u = h >> 2, ph = h & 3;
+                f.fft(sm, lay, bar, t, opaque(tw));
+                f.scale(sm, lay, bar, t);
+                const bool last = u == nsub - 1;
+                if ((ph & 1) == 0) {
+                    f.ex += a.hs_exp;
+                    f.mul([&](int e) { return __ldg(tab(hs) + e * TL); }, false);
+                    f.conj();
+                } else if (ph == 1) {
+                    const fixw *k = tab(a.order == 4 && u == 1 ? k1 : k0);
+                    f.ex += a.k_exp;
+                    f.conj();
+                    f.mul([&](int e) { return __ldg(k + e * TL); }, false);
+                    f.conj();
+                } else {
+                    f.mul(upto_n(tab(a.order == 4 && !last ? v1 : v0)), last && s + 1 < a.nsteps);
+                }
+            }
+        }
+        if (a.nsteps) {
+            f.conj();
+            f.mul([&](int e) { return __ldg(tab(w) + e * TL); }, false);
+            f.conj();
+        }
+        f.store(x);
+    } else {
     apply_v(v0, false);
 #pragma unroll 1
     for (uint64_t s = 0; s < a.nsteps; ++s) {
@@ -123,6 +171,7 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
             const bool last = u == nsub - 1;
             apply_v((a.order == 4 && !last) ? v1 : v0, last && s + 1 < a.nsteps);
         }
+    }
     }
     double nsum = 0;
     const int nn = a.norm_n ? a.norm_n : n;
@@ -226,6 +275,9 @@ struct Blue2DArgs {
     const void *w, *hs;     // Bluestein tables of this pass's side (M entries)
     const void *kx, *ky;    // column pass: kinetic factors along x (nx entries, 1/(nx ny) folded) and y
     int nx, ny;
+    // complex128, real time steps: fixed-point tables (fixw) in their place; the values of hs
+    // and kx are the tables' times 2^hs_exp and 2^k_exp
+    int fx, hs_exp, k_exp;
 };
 
 // one DFT of the M-slot line x (zero above the side length): forward when
@@ -256,9 +308,11 @@ __device__ __forceinline__ void blue_dft(C (&x)[E], C *sm, const Lay &lay, const
     }
 }
 
-// Row pass: RPC rows per CTA, TL = M / E threads per row.
-template <class T, int M, int E, int RPC>
-__global__ void __launch_bounds__(RPC *(M / E)) k_row_blue(Blue2DArgs a)
+// Row pass: RPC rows per CTA, TL = M / E threads per row.  FX (complex128, real
+// time steps): one trip to fixed point per pass, the chirps around V cancelled.
+template <class T, int M, int E, int RPC, bool FX = false>
+__global__ void __launch_bounds__(RPC *(M / E), FX && RPC * (M / E) <= 256 ? 768 / (RPC * (M / E)) : 0)
+    k_row_blue(Blue2DArgs a)
 {
     using C = cplx_t<T>;
     constexpr int TL = M / E;
@@ -281,6 +335,44 @@ __global__ void __launch_bounds__(RPC *(M / E)) k_row_blue(Blue2DArgs a)
         const int j = t + e * TL;
         x[e] = j < ny ? psi[j] : cmk<C>(0, 0);
     }
+    if constexpr (FX) {
+        const fixw *wf = reinterpret_cast<const fixw *>(w) + t, *hf = reinterpret_cast<const fixw *>(hs) + t;
+        const fixw *vt = static_cast<const fixw *>(a.vtab);
+        const bool bad = vt && fix_flagged(vt + (size_t)a.nx * ny);
+        const fixw *vr = vt + (size_t)(active ? row : 0) * ny + t;
+        FixLine<M, E> f;
+        f.load(x, sm, lay, bar, t);
+        if (bad) f.finite = false;
+        if (a.in_k) {
+            f.conj();
+            f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+        }
+        const int npass = 2 * ((a.in_k ? 1 : 0) + (a.out_k ? 1 : 0)), vpos = a.in_k ? 2 : 0;
+#pragma unroll 1
+        for (int p = 0; p <= npass; ++p) {
+            if (p > 0) f.scale(sm, lay, bar, t);
+            if (p == vpos) {
+                if (a.in_k && !a.out_k) {  // the inverse DFT's closing w* (out_k: cancels against the opening w)
+                    f.conj();
+                    f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+                    f.conj();
+                }
+                if (vt)
+                    f.mul([&](int e) { return t + e * TL < ny ? ld_stream(vr + e * TL) : fixw{0, 0, 0, 0}; },
+                          a.vtwice != 0);
+                if (a.out_k && !a.in_k) f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+            } else if (p & 1) {
+                f.ex += a.hs_exp;
+                f.mul([&](int e) { return __ldg(hf + e * TL); }, false);
+                f.conj();
+            } else if (p == npass) {
+                f.conj();
+                f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+            }
+            if (p < npass) f.fft(sm, lay, bar, t, opaque(tw));
+        }
+        f.store(x);
+    } else {
     if (a.in_k) {
         blue_dft<true, C, M, E>(x, sm, lay, bar, t, tw, w, hs);
     }
@@ -302,6 +394,7 @@ __global__ void __launch_bounds__(RPC *(M / E)) k_row_blue(Blue2DArgs a)
             if (t + e * TL >= ny) x[e] = cmk<C>(0, 0);
         blue_dft<false, C, M, E>(x, sm, lay, bar, t, tw, w, hs);
     }
+    }
     if (active) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
@@ -311,9 +404,11 @@ __global__ void __launch_bounds__(RPC *(M / E)) k_row_blue(Blue2DArgs a)
     }
 }
 
-// Column pass: W adjacent columns per CTA, TM = M / E threads per column.
-template <class T, int M, int E, int W>
-__global__ void __launch_bounds__(W *(M / E)) k_col_blue(Blue2DArgs a)
+// Column pass: W adjacent columns per CTA, TM = M / E threads per column.  FX as
+// in the row pass: the chirps around K cancel (K then applies conjugated).
+template <class T, int M, int E, int W, bool FX = false>
+__global__ void __launch_bounds__(W *(M / E), FX && W * (M / E) <= 512 ? 1024 / (W * (M / E)) : 0)
+    k_col_blue(Blue2DArgs a)
 {
     using C = cplx_t<T>;
     constexpr int TM = M / E;
@@ -337,6 +432,35 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_blue(Blue2DArgs a)
         const int i = t + e * TM;
         x[e] = i < nx ? psi[(size_t)i * ny] : cmk<C>(0, 0);
     }
+    if constexpr (FX) {
+        const fixw *wf = reinterpret_cast<const fixw *>(w) + t, *hf = reinterpret_cast<const fixw *>(hs) + t;
+        const fixw *kx = static_cast<const fixw *>(a.kx) + t;
+        const fixw kyf = __ldg(static_cast<const fixw *>(a.ky) + (active ? col : 0));
+        FixLine<M, E> f;
+        f.load(x, sm, lay, bar, t);
+        f.mul([&](int e) { return __ldg(wf + e * TM); }, false);
+#pragma unroll 1
+        for (int p = 0; p < 4; ++p) {
+            f.fft(sm, lay, bar, t, opaque(tw));
+            f.scale(sm, lay, bar, t);
+            if ((p & 1) == 0) {
+                f.ex += a.hs_exp;
+                f.mul([&](int e) { return __ldg(hf + e * TM); }, false);
+                f.conj();
+            } else if (p == 1) {
+                f.ex += a.k_exp;
+                f.conj();
+                f.mul([&](int e) { return t + e * TM < nx ? __ldg(kx + e * TM) : fixw{0, 0, 0, 0}; }, false);
+                f.mul([&](int) { return kyf; }, false);
+                f.conj();
+            } else {
+                f.conj();
+                f.mul([&](int e) { return __ldg(wf + e * TM); }, false);
+                f.conj();
+            }
+        }
+        f.store(x);
+    } else {
     blue_dft<false, C, M, E>(x, sm, lay, bar, t, tw, w, hs);
     const C ky = ld_c(static_cast<const C *>(a.ky) + (active ? col : 0));
 #pragma unroll
@@ -345,6 +469,7 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_blue(Blue2DArgs a)
         x[e] = i < nx ? cmul(cmul(x[e], ld_c(static_cast<const C *>(a.kx) + i)), ky) : cmk<C>(0, 0);
     }
     blue_dft<true, C, M, E>(x, sm, lay, bar, t, tw, w, hs);
+    }
     if (active) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {

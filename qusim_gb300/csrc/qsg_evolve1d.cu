@@ -12,14 +12,17 @@ bool evolve1d_supported(int prec, uint64_t n)
 }
 constexpr int res_ni_for(int l, int e) { return (256 / (l / e)) > 1 ? 256 / (l / e) : 1; }
 
-template <class T, int L>
+template <class T, int L, bool FX = false>
 static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_evolve1d<T, L, true>(a, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     constexpr int NI = res_ni_for(L, E);
     const size_t smem = sizeof(cplx_t<T>) * padded<L, PADS>(L) * NI;
-    auto k = k_evolve1d_resident<T, L, E, NI>;
+    auto k = k_evolve1d_resident<T, L, E, NI, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<(a.count + NI - 1) / NI, NI * (L / E), smem, st>>>(a);
@@ -103,13 +106,16 @@ bool wall1d_supported(int prec, uint64_t n)
     return prec == 1 ? 2 * n <= 8192 : 2 * n <= 4096;
 }
 
-template <class T, int L2>
+template <class T, int L2, bool FX = false>
 static cudaError_t run_wall(const Evolve1DBatchArgs &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_wall<T, L2, true>(a, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * padded<L2, PADS>(L2);
-    auto k = k_evolve1d_wall<T, L2, E>;
+    auto k = k_evolve1d_wall<T, L2, E, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<a.count, L2 / E, smem, st>>>(a);
@@ -201,26 +207,32 @@ bool fs_geom(int prec, uint64_t n, FsGeom *g, int n1)
     return g->col_blocks >= 1 && g->row_blocks >= 1;
 }
 
-template <class T, int N2>
+template <class T, int N2, bool FX = false>
 static cudaError_t run_fs_col(const FsGeom &g, const FsColArgs &a, int ninst, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_fs_col<T, N2, true>(g, a, ninst, st);
+    }
     constexpr int P = sizeof(T) == 4 ? 1 : 0;
     constexpr int E = P ? 16 : 8;
     constexpr int W = fs_col_w(P, N2);
-    auto k = k_fs_col<T, N2, E, W>;
+    auto k = k_fs_col<T, N2, E, W, FX>;
     cudaError_t e = prepare_smem(k, g.col_smem);
     if (e != cudaSuccess) return e;
     k<<<dim3(g.col_blocks, ninst), W * (N2 / E), g.col_smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <class T, int N1>
+template <class T, int N1, bool FX = false>
 static cudaError_t run_fs_row(const FsGeom &g, const FsRowArgs &a, int ninst, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_fs_row<T, N1, true>(g, a, ninst, st);
+    }
     constexpr int P = sizeof(T) == 4 ? 1 : 0;
     constexpr int E = P ? 16 : 8;
     constexpr int B = fs_row_b(P, N1);
-    auto k = k_fs_row<T, N1, E, B>;
+    auto k = k_fs_row<T, N1, E, B, FX>;
     cudaError_t e = prepare_smem(k, g.row_smem);
     if (e != cudaSuccess) return e;
     k<<<dim3(g.row_blocks, ninst), B * (N1 / E), g.row_smem, st>>>(a);

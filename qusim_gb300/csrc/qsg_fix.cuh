@@ -126,15 +126,15 @@ template <int TL, class Lay, int OP> struct FixReduce {
     }
 };
 
-// the double d as units of 2^(emax - 1023 - 58): its 53-bit significand from bit 58 down,
-// shifted by the distance of its exponent from emax (magnitude bits below the unit dropped)
-__device__ __forceinline__ long long fix_from(double d, int emax)
+// the double d as units of 2^(emax - 1023 - 52 - up): its 53-bit significand from bit 52 + up
+// down, shifted by the distance of its exponent from emax (magnitude bits below the unit dropped)
+__device__ __forceinline__ long long fix_from(double d, int emax, int up = 6)
 {
     const int hi = __double2hiint(d);
     const unsigned lo = (unsigned)__double2loint(d);
     const int e = (hi >> 20) & 0x7ff;
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const unsigned long long m = ((unsigned long long)mh << 32 | lo) << 6;
+    const unsigned long long m = ((unsigned long long)mh << 32 | lo) << up;
     int sh = emax - e;
     sh = sh > 63 ? 63 : sh;
     const long long v = (long long)(m >> sh);
@@ -311,19 +311,20 @@ template <int L, int E> struct FixLine {
         fix_norm(v, Red::get(m, w + r), ex);
         if constexpr (!Red::WARP) r = after(r);
     }
-    // v *= f(e), `twice`: two products (the reference's two multiplies by one table value)
-    template <class F> __device__ __forceinline__ void mul(F f, bool twice)
+    // v *= f(e), `twice`: two products (the reference's two multiplies by one table value);
+    // H < E: only the first H slots (the others are not used afterwards)
+    template <int H = E, class F> __device__ __forceinline__ void mul(F f, bool twice)
     {
         if (twice) {
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
+            for (int e = 0; e < H; ++e) {
                 const fixw m = f(e);
                 v[e] = fix_twmul(fix_twmul(v[e], m), m);
             }
             ex += 4;
         } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = fix_twmul(v[e], f(e));
+            for (int e = 0; e < H; ++e) v[e] = fix_twmul(v[e], f(e));
             ex += 2;
         }
     }

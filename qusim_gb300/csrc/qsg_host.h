@@ -119,16 +119,18 @@ inline int dev_alloc(qsg_ctx *ctx, size_t bytes, void **p, size_t *acct, bool bu
 // 2 complex64 plain (float2, each factor rounded once), 3 fixed point (fixw, qsg_fix.cuh)
 inline size_t twsize(int prec) { return prec == 2 ? 8 : 16; }
 
-// |v| <= 1 as hi 2^-30 + lo 2^-62 (lo kept within +-(2^31 - 1), so both words can be negated)
+// v1 + v2 (v2 the rest of a value below v1's last place), |v1 + v2| <= 1, as hi 2^-30 + lo 2^-62;
+// lo is kept within +-(2^31 - 1), so both words can be negated
+inline void put_fixed(double v1, double v2, int32_t *hi, int32_t *lo)
+{
+    const double s = v1 * 0x1p30, h = std::nearbyint(s), l = std::nearbyint((s - h) * 0x1p32 + v2 * 0x1p62);
+    *hi = (int32_t)h;
+    *lo = (int32_t)(l > 2147483647.0 ? 2147483647.0 : (l < -2147483647.0 ? -2147483647.0 : l));
+}
 inline void put_fixed(long double v, int32_t *hi, int32_t *lo)
 {
-    const long double s = v * 1073741824.0L;
-    const long double h = roundl(s);
-    long double l = roundl((s - h) * 4294967296.0L);
-    if (l > 2147483647.0L) l = 2147483647.0L;
-    if (l < -2147483647.0L) l = -2147483647.0L;
-    *hi = (int32_t)h;
-    *lo = (int32_t)l;
+    const double v1 = (double)v;
+    put_fixed(v1, (double)(v - (long double)v1), hi, lo);
 }
 
 inline void put_twiddle(int prec, unsigned char *dst, long double re, long double im)

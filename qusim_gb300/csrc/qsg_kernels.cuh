@@ -143,7 +143,7 @@ struct Evolve1DBatchArgs;
 // NI instances per CTA (instance blockIdx.x*NI + line); all instances of one
 // launch share N and the order.  V tables vtab[0..1], kinetic tables ktab[0..1] (natural layout,
 // 1/N folded in for complex128, factor - 1 for complex64).
-template <class T, int L, int E, int NI>
+template <class T, int L, int E, int NI, bool FX = false>
 __global__ void __launch_bounds__(NI *(L / E)) k_evolve1d_resident(Evolve1DBatchArgs a);
 
 // ---------------------------------------------------------------------------
@@ -434,7 +434,7 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
 // complex128 runs at three CTAs of 256 threads per SM (85 registers): with two
 // (126) its integer pipes wait more (1024^2: 51.5 -> 43.3 us per launch).
 template <class T, int NY, int E, int G, int B, int RS, bool PL = false, bool FX = false>
-__global__ void __launch_bounds__(B *G *(NY / E) / RS, sizeof(T) == 8 && G == 1 ? 768 / (B * G * (NY / E) / RS) : 1)
+__global__ void __launch_bounds__(B *G *(NY / E) / RS, sizeof(T) == 8 ? (G == 1 ? 768 : 512) / (B * G * (NY / E) / RS) : 0)
     k_row_pass(RowPassArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -736,6 +736,7 @@ struct FsColArgs {
     int n1;
     int vsel, vtwice;       // V table index; apply it twice
     int in_k, out_k;        // input in k layout / output to k layout
+    int fx;                 // complex128: vtab and tw_n hold fixed-point factors
     const void *maps;       // tensor-copy pass: 3 tensor maps per instance (state, V 0, V 1), or null
     int tiles;              // tensor-copy pass: column blocks x instances
     int *err;               // tensor-copy pass: counter it adds 1 to when a bounded wait ran out
@@ -747,8 +748,11 @@ struct FsColArgs {
 
 // three 256-thread CTAs per SM (registers capped at 85) for the strided
 // column pass: it waits on its scattered loads more than it issues
-template <class T, int N2, int E, int W>
-__global__ void __launch_bounds__(W *(N2 / E), (W * (N2 / E) <= 256 && sizeof(T) == 4) ? 3 : 1) k_fs_col(FsColArgs a)
+// FX (complex128, real time steps): twiddles, transforms and potential products
+// in fixed point
+template <class T, int N2, int E, int W, bool FX = false>
+__global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T) == 4 || FX) ? 768 / (W * (N2 / E)) : 1)
+    k_fs_col(FsColArgs a)
 {
     using C = cplx_t<T>;
     constexpr int TM = Plan<N2, E>::TL;
@@ -777,6 +781,47 @@ __global__ void __launch_bounds__(W *(N2 / E), (W * (N2 / E) <= 256 && sizeof(T)
 #pragma unroll
         for (int e = 0; e < E; ++e) x[e] = ld_stream(p + e * stride);
     }
+    double nsum = 0;
+    if constexpr (FX) {
+        const fixw *wn = reinterpret_cast<const fixw *>(twn) + base;
+        const fixw *vt = static_cast<const fixw *>((a.vsel ? in.vtab[1] : in.vtab[0]));
+        FixLine<N2, E> f;
+        f.load(x, sm, lay, bar, t);
+        if (vt && fix_flagged(vt + (size_t)N2 * n1)) f.finite = false;
+        if (in_k) {
+            f.conj();
+            f.mul([&](int e) { return __ldg(wn + e * stride); }, false);
+        }
+        const int npass = (in_k ? 1 : 0) + (out_k ? 1 : 0);
+        const int vpos = in_k ? 1 : 0;
+#pragma unroll 1
+        for (int p = 0; p <= npass; ++p) {
+            if (p == vpos) {
+                if (in_k) {
+                    f.conj();
+                    f.scale(sm, lay, bar, t);
+                }
+                if (vt) {
+                    const fixw *vr = opaque(vt) + base;
+                    f.mul([&](int e) { return ld_stream(vr + e * stride); }, a.vtwice != 0);
+                } else {
+                    f.quarter();
+                }
+                if (a.wall && out_k && col == 0 && t == 0) f.v[0] = f.v[E / 2] = Fix{0, 0};
+            }
+            if (p < npass) f.fft(sm, lay, bar, t, opaque(tw));
+        }
+        if (out_k) {
+            f.scale(sm, lay, bar, t);
+            const fixw *wo = opaque(wn);
+            f.mul([&](int e) { return __ldg(wo + e * stride); }, false);
+        }
+        f.store(x);
+        if (!out_k) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) nsum += abs2d(x[e]);
+        }
+    } else {
     if (in_k) {
         // iFFT(y * conj(w)) = conj(FFT(conj(y) * w))
 #pragma unroll
@@ -813,13 +858,13 @@ __global__ void __launch_bounds__(W *(N2 / E), (W * (N2 / E) <= 256 && sizeof(T)
         }
         if (p < npass) line_fft<C, N2, E, false>(x, sm, lay, bar, t, tw);
     }
-    double nsum = 0;
     if (out_k) {
 #pragma unroll
         for (int e = 0; e < E; ++e) x[e] = twmul<false>(x[e], __ldg(opaque(twn) + base + e * stride));
     } else {
 #pragma unroll
         for (int e = 0; e < E; ++e) nsum += abs2d(x[e]);
+    }
     }
     {
         C *p = const_cast<C *>(opaque(psi)) + base;
@@ -839,11 +884,14 @@ struct FsRowArgs {
     float inv_n;            // 1/N (complex64 path; complex128 tables carry it)
     int plain;              // the table holds plain complex factors (any modulus, scale included):
                             // a plain product, no 1/N (Bluestein's convolution kernels)
+    int fx;                 // complex128: the tables hold fixed-point factors ...
+    int kexp[2];            // ... times 2^kexp[ksel] (1/N, or the scale of a convolution kernel)
 };
 
-// B rows of N1 per CTA (B * N1/E threads)
-template <class T, int N1, int E, int B>
-__global__ void __launch_bounds__(B *(N1 / E)) k_fs_row(FsRowArgs a)
+// B rows of N1 per CTA (B * N1/E threads).  FX as in k_fs_col.
+template <class T, int N1, int E, int B, bool FX = false>
+__global__ void __launch_bounds__(B *(N1 / E), FX && B * (N1 / E) <= 256 ? 768 / (B * (N1 / E)) : 0)
+    k_fs_row(FsRowArgs a)
 {
     using C = cplx_t<T>;
     constexpr int TL = Plan<N1, E>::TL;
@@ -865,6 +913,22 @@ __global__ void __launch_bounds__(B *(N1 / E)) k_fs_row(FsRowArgs a)
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = ld_stream(psi + base + e * TL);
     // FFT -> K -> iFFT, the iFFT as conj(FFT(conj(x)))
+    if constexpr (FX) {
+        FixLine<N1, E> f;
+        f.load(x, sm, lay, lbar, t);
+        f.ex += (a.ksel ? a.kexp[1] : a.kexp[0]);
+#pragma unroll 1
+        for (int p = 0; p < 2; ++p) {
+            f.fft(sm, lay, lbar, t, opaque(tw));
+            if (p == 0) {
+                f.scale(sm, lay, lbar, t);
+                const fixw *kt = opaque(static_cast<const fixw *>((a.ksel ? in.ktab[1] : in.ktab[0]))) + base;
+                f.mul([&](int e) { return ld_stream(kt + e * TL); }, false);
+            }
+            if (p == 0) f.conj();
+        }
+        f.store(x);
+    } else {
 #pragma unroll 1
     for (int p = 0; p < 2; ++p) {
         line_fft<C, N1, E, false>(x, sm, lay, lbar, t, tw);
@@ -881,6 +945,7 @@ __global__ void __launch_bounds__(B *(N1 / E)) k_fs_row(FsRowArgs a)
                 x[e] = cconj(PhaseOps<C>::apply(v, ld_stream(kt + e * TL)));
             }
         }
+    }
     }
     C *p = const_cast<C *>(opaque(psi)) + base;
 #pragma unroll
@@ -939,12 +1004,14 @@ struct Evolve1DBatchArgs {
     uint64_t nsteps;
     int order, renormalize;
     int count;              // instances in the launch
+    int fx;                 // complex128: the phase tables hold fixed-point factors
 };
 
 // The lines of NI instances of length L, held by the NI * (L / E) threads of
 // the CTA: instance `first + line` for line < count (the other lines run on
 // instance `first` without storing), for all a.nsteps steps.
-template <class T, int L, int E, int NI>
+// FX (complex128, real time steps): the line stays in fixed point for all of them.
+template <class T, int L, int E, int NI, bool FX = false>
 __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int first, int count, const void *twp,
                                                unsigned char *smraw)
 {
@@ -981,6 +1048,30 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
     // one count for the whole launch: instances that share a CTA synchronise
     // with CTA-wide barriers, so every line must run the same number of steps
     const uint64_t nsteps = a.nsteps;
+    if constexpr (FX) {
+        FixLine<L, E> f;
+        f.load(x, sm, lay, bar, t);
+        auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
+        if (fix_flagged(tab(v0) - t + L) || (a.order == 4 && fix_flagged(tab(v1) - t + L))) f.finite = false;
+        f.mul([&](int e) { return __ldg(tab(v0) + e * TL); }, false);
+        for (uint64_t s = 0; s < nsteps; ++s) {
+#pragma unroll 1
+            for (int h = 0; h < 2 * nsub; ++h) {
+                f.fft(sm, lay, bar, t, opaque(tw));
+                f.scale(sm, lay, bar, t);
+                const int u = h >> 1;
+                const bool last = u == nsub - 1, kin = (h & 1) == 0;
+                const fixw *m = tab(kin ? (a.order == 4 && u == 1 ? k1 : k0) : (a.order == 4 && !last ? v1 : v0));
+                if (kin)
+                    f.ex -= Plan<L, E>::LOGL;  // 1/N
+                else
+                    f.conj();
+                f.mul([&](int e) { return __ldg(m + e * TL); }, !kin && last && s + 1 < nsteps);
+                if (kin) f.conj();
+            }
+        }
+        f.store(x);
+    } else {
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = PhaseOps<C>::apply(x[e], ld_c(v0 + t + e * TL));
     for (uint64_t s = 0; s < nsteps; ++s) {
@@ -1009,6 +1100,7 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
                 }
             }
         }
+    }
     }
 
     if (a.norm_out || a.renormalize) {
@@ -1045,12 +1137,12 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
     }
 }
 
-template <class T, int L, int E, int NI>
+template <class T, int L, int E, int NI, bool FX>
 __global__ void __launch_bounds__(NI *(L / E)) k_evolve1d_resident(Evolve1DBatchArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int first = blockIdx.x * NI;
-    evolve1d_lines<T, L, E, NI>(a, first, a.count - first, a.tw, smraw);
+    evolve1d_lines<T, L, E, NI, FX>(a, first, a.count - first, a.tw, smraw);
 }
 
 // One persistent launch over the resident-size classes of a batch with
@@ -1136,7 +1228,8 @@ __device__ __forceinline__ void odd_extend(C (&x)[E], C *sm, const Lay &lay, int
     if (t == 0) x[0] = cmk<C>(0, 0);
 }
 
-template <class T, int L2, int E>
+// FX (complex128, real time steps): the line stays in fixed point for all of them
+template <class T, int L2, int E, bool FX = false>
 __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
 {
     using C = cplx_t<T>;
@@ -1164,6 +1257,30 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
 
     const int nsub = a.order == 2 ? 1 : 3;
     const uint64_t nsteps = a.nsteps;
+    if constexpr (FX) {
+        FixLine<L2, E> f;
+        f.load(x, sm, lay, bar, t);
+        auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
+        if (fix_flagged(tab(v0) - t + L2 / 2) || (a.order == 4 && fix_flagged(tab(v1) - t + L2 / 2))) f.finite = false;
+        f.template mul<H>([&](int e) { return __ldg(tab(v0) + e * TL); }, false);
+        for (uint64_t s = 0; s < nsteps; ++s) {
+#pragma unroll 1
+            for (int h = 0; h < 2 * nsub; ++h) {
+                // two inverse transforms of odd extensions, K between them
+                odd_extend<Fix, L2, E>(f.v, reinterpret_cast<Fix *>(sm), lay, t);
+                f.conj();
+                f.fft(sm, lay, bar, t, opaque(tw));
+                f.conj();
+                f.scale(sm, lay, bar, t);
+                const int u = h >> 1;
+                const bool last = u == nsub - 1, kin = (h & 1) == 0;
+                const fixw *m = tab(kin ? (a.order == 4 && u == 1 ? k1 : k0) : (a.order == 4 && !last ? v1 : v0));
+                if (kin) f.ex -= Plan<L2, E>::LOGL;  // 1/(2N); the table carries the sign
+                f.template mul<H>([&](int e) { return __ldg(m + e * TL); }, !kin && last && s + 1 < nsteps);
+            }
+        }
+        f.store(x);
+    } else {
 #pragma unroll
     for (int e = 0; e < H; ++e) x[e] = PhaseOps<C>::apply(x[e], ld_c(v0 + t + e * TL));
     for (uint64_t s = 0; s < nsteps; ++s) {
@@ -1196,6 +1313,7 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
                 if (twice) x[e] = PhaseOps<C>::apply(x[e], m);
             }
         }
+    }
     }
     if (a.norm_out || a.renormalize) {
         double sum = 0;

@@ -87,3 +87,63 @@ def test_columns_of_very_different_size_vs_oracle(qsg, ctx, oracle, shape):
     inst = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, 0.01, order=4)
     inst.step(2)
     assert rel_l2(inst.get_psi(), ref) <= TOL
+
+
+# one CTA, Bluestein, four-step, Bluestein on the four-step passes; walls
+@pytest.mark.parametrize("n,wall", [(64, 0), (4096, 0), (1000, 0), (16384, 0), (6000, 0), (512, 1), (700, 1), (4096, 1)])
+def test_infinite_potential_gives_nan(qsg, ctx, n, wall):
+    psi, V = line(n, "noise")
+    V[n // 2] = np.inf
+    inst = qsg.Instance.create_1d(ctx, psi, V, 0.1, 0.01, order=4,
+                                  boundary=qsg.BoundaryCondition.InfiniteWall if wall else qsg.BoundaryCondition.Period)
+    inst.step(1)
+    got = inst.get_psi()
+    assert not np.isfinite(got[1:]).any()
+
+
+@pytest.mark.parametrize("shape", [(128, 128), (512, 256), (30, 45)])
+def test_infinite_potential_gives_nan_2d(qsg, ctx, shape):
+    rng = np.random.default_rng(2)
+    psi = rng.standard_normal(shape) + 0j
+    V = rng.uniform(-1, 1, shape)
+    V[3, 5] = np.inf
+    inst = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, 0.01, order=2)
+    inst.step(1)
+    assert not np.isfinite(inst.get_psi()).any()
+
+
+@pytest.mark.parametrize("n", [256, 16384])
+def test_batch_of_real_and_complex_steps_equals_solo(qsg, ctx, n):
+    # real time steps run in fixed point, complex ones in double: two classes of one length
+    psis, Vs = zip(*(line(n, "noise", seed) for seed in range(4)))
+    dts = [0.01, 0.01 - 0.002j, 0.02, -0.005j]
+    b = qsg.Batch(ctx, psis, Vs, [0.1] * 4, dts, order=2)
+    if n > 4096:
+        plan = next(p for p in qsg.candidate_plans_1d("fp64", n) if p.kind == 1 and p.n1 != b.plan(n).n1)
+        b.set_plan(n, plan)
+    b.step(5)
+    for i in range(4):
+        solo = qsg.Instance.create_1d(ctx, psis[i], Vs[i], 0.1, dts[i], order=2)
+        if n > 4096:
+            solo.set_plan(plan)
+        solo.step(5)
+        assert np.array_equal(b.instance(i).get_psi(), solo.get_psi()), i
+
+
+@pytest.mark.parametrize("shape", [(128, 128), (1024, 256), (4096, 128), (256, 512)])
+def test_every_2d_plan_vs_oracle(qsg, ctx, oracle, shape):
+    # four and eight elements a thread, units of fewer threads, unsplit columns up to 4096, both
+    # with fixed-point products (real steps) and double ones (complex steps)
+    nx, ny = shape
+    rng = np.random.default_rng(4)
+    psi = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    V = rng.uniform(-1, 1, shape)
+    for dt in (0.01, 0.01 - 0.0005j):
+        ref = oracle.evolve2d(psi, V, 0.1, 0.1, dt, 1, order=2)
+        inst = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, dt, order=2)
+        for plan in inst.candidate_plans():
+            inst.set_psi(psi)
+            inst.set_plan(plan)
+            inst.step(1)
+            got = inst.get_psi()
+            assert rel_l2(got, ref) <= TOL, (dt, plan.g, plan.row_e, plan.row_nt, plan.col_e, plan.col_w)
