@@ -1,7 +1,7 @@
 // qsg_aux.cu -- phase tables, reductions, conversions.
 #include "qsg_aux.h"
 #include <type_traits>
-#include "qsg_kernels.cuh"
+#include "qsg_dispatch.cuh"
 
 namespace qsg {
 
@@ -181,6 +181,7 @@ __global__ void k_ktable2d(C *out, int nx, int ny, double are, double aim, doubl
 
 __global__ void k_c128_to_c64(float2 *out, const double2 *in, size_t n)
 {
+    pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double2 v = in[i];
         out[i] = make_float2(float(v.x), float(v.y));
@@ -188,6 +189,7 @@ __global__ void k_c128_to_c64(float2 *out, const double2 *in, size_t n)
 }
 __global__ void k_c64_to_c128(double2 *out, const float2 *in, size_t n)
 {
+    pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float2 v = in[i];
         out[i] = make_double2(double(v.x), double(v.y));
@@ -236,6 +238,7 @@ template <class C, int MODE>
 __global__ void __launch_bounds__(kThreads) k_reduce(const C *__restrict__ psi, const double *__restrict__ V,
                                                      size_t lo, size_t hi, double *partials)
 {
+    pdl_wait();
     __shared__ double red[32];
     double s = 0;
     SumF2 f;
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(kThreads) k_reduce(const C *__restrict__ psi, 
 __global__ void __launch_bounds__(kThreads) k_finalize(const double *partials, int nparts, int stride,
                                                        double *out)
 {
+    pdl_wait();
     __shared__ double red[32];
     for (int k = 0; k < stride; ++k) {
         double s = 0;
@@ -270,6 +274,7 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const double *partials, i
 template <class C, class T>
 __global__ void k_renorm(C *psi, size_t n, const double *sum, double dv)
 {
+    pdl_wait();
     const T sc = T(1.0 / sqrt(sum[0] * dv));
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         C v = psi[i];
@@ -379,13 +384,13 @@ cudaError_t launch_ktable2d(int prec, void *out, int nx, int ny, double are, dou
 
 cudaError_t launch_c128_to_c64(void *out, const void *in, size_t n, cudaStream_t st)
 {
-    k_c128_to_c64<<<blocks_for(n), kThreads, 0, st>>>((float2 *)out, (const double2 *)in, n);
+    launch_pdl(k_c128_to_c64, dim3(blocks_for(n)), dim3(kThreads), 0, st, (float2 *)out, (const double2 *)in, n);
     return cudaGetLastError();
 }
 
 cudaError_t launch_c64_to_c128(void *out, const void *in, size_t n, cudaStream_t st)
 {
-    k_c64_to_c128<<<blocks_for(n), kThreads, 0, st>>>((double2 *)out, (const float2 *)in, n);
+    launch_pdl(k_c64_to_c128, dim3(blocks_for(n)), dim3(kThreads), 0, st, (double2 *)out, (const float2 *)in, n);
     return cudaGetLastError();
 }
 
@@ -397,7 +402,7 @@ cudaError_t launch_reduce(int prec, const void *psi, const double *V, size_t lo,
     if (b > 1216) b = 1216;
     if ((int)b > max_parts) b = (unsigned)max_parts;
     *nparts = (int)b;
-#define QSG_REDUCE(C, M) k_reduce<C, M><<<b, kThreads, 0, st>>>((const C *)psi, V, lo, hi, partials)
+#define QSG_REDUCE(C, M) launch_pdl(k_reduce<C, M>, dim3(b), dim3(kThreads), 0, st, (const C *)psi, V, lo, hi, partials)
     if (prec == 1) {
         if (mode == 0) QSG_REDUCE(float2, 0);
         else if (mode == 1) QSG_REDUCE(float2, 1);
@@ -414,16 +419,16 @@ cudaError_t launch_reduce(int prec, const void *psi, const double *V, size_t lo,
 cudaError_t launch_finalize(const double *partials, int nparts, int stride, double *out,
                             cudaStream_t st)
 {
-    k_finalize<<<1, kThreads, 0, st>>>(partials, nparts, stride, out);
+    launch_pdl(k_finalize, dim3(1), dim3(kThreads), 0, st, partials, nparts, stride, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_renorm(int prec, void *psi, size_t n, const double *sum, double dv, cudaStream_t st)
 {
     if (prec == 1)
-        k_renorm<float2, float><<<blocks_for(n), kThreads, 0, st>>>((float2 *)psi, n, sum, dv);
+        launch_pdl(k_renorm<float2, float>, dim3(blocks_for(n)), dim3(kThreads), 0, st, (float2 *)psi, n, sum, dv);
     else
-        k_renorm<double2, double><<<blocks_for(n), kThreads, 0, st>>>((double2 *)psi, n, sum, dv);
+        launch_pdl(k_renorm<double2, double>, dim3(blocks_for(n)), dim3(kThreads), 0, st, (double2 *)psi, n, sum, dv);
     return cudaGetLastError();
 }
 

@@ -27,7 +27,7 @@ cudaError_t run_blue(const BlueArgs &a, cudaStream_t st)
     auto k = k_evolve1d_blue<T, M, E, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<1, M / E, smem, st>>>(a);
+    launch_pdl(k, dim3(1), dim3(M / E), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -289,7 +289,7 @@ cudaError_t run_row_blue(const Blue2DArgs &a, cudaStream_t st)
     auto k = k_row_blue<T, M, E, RPC, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(a.nx + RPC - 1) / RPC, RPC * (M / E), smem, st>>>(a);
+    launch_pdl(k, dim3((a.nx + RPC - 1) / RPC), dim3(RPC * (M / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -315,12 +315,12 @@ cudaError_t run_col_blue(const Blue2DArgs &a, bool kinetic, double dtx, double d
         auto k = k_col_blue<T, M, E, W, sizeof(T) == 8>;
         cudaError_t e = prepare_smem(k, smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, W * (M / E), smem, st>>>(a);
+        launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a);
     } else {
         auto k = k_col_blue<T, M, E, W>;
         cudaError_t e = prepare_smem(k, smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, W * (M / E), smem, st>>>(a);
+        launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a);
     }
     return cudaGetLastError();
 }

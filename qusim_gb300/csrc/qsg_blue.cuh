@@ -59,6 +59,7 @@ struct BlueArgs {
 template <class T, int M, int E, bool FX = false>
 __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = M / E;
     constexpr int PADS = sizeof(C) == 8 ? 4 : 3;
@@ -314,6 +315,7 @@ template <class T, int M, int E, int RPC, bool FX = false>
 __global__ void __launch_bounds__(RPC *(M / E), FX && RPC * (M / E) <= 256 ? 768 / (RPC * (M / E)) : 0)
     k_row_blue(Blue2DArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = M / E;
     constexpr int PADS = sizeof(C) == 8 ? 4 : 3;
@@ -410,6 +412,7 @@ template <class T, int M, int E, int W, bool FX = false>
 __global__ void __launch_bounds__(W *(M / E), FX && W * (M / E) <= 512 ? 1024 / (W * (M / E)) : 0)
     k_col_blue(Blue2DArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TM = M / E;
     extern __shared__ __align__(16) unsigned char smraw[];

@@ -140,6 +140,7 @@ constexpr int born_min_blocks(int threads) { return threads <= 256 ? 2 : 1; }
 template <class T, int NY, int E, int G, int B>
 __global__ void __launch_bounds__(B *G *(NY / E), born_min_blocks(B *G *(NY / E))) k_born_row(BornRowArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = Plan<NY, E>::TL;
     constexpr int NL = B * G;
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(B *G *(NY / E), born_min_blocks(B *G *(NY / E)
 template <class T, int M, int E, int W>
 __global__ void __launch_bounds__(W *(M / E), born_min_blocks(W *(M / E))) k_born_col(BornColArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TM = Plan<M, E>::TL;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(W *(M / E), born_min_blocks(W *(M / E))) k_bor
 template <class T, int L, int E>
 __global__ void __launch_bounds__(L / E) k_born1d(Born1DArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = Plan<L, E>::TL;
     constexpr int PADS = sizeof(C) == 8 ? 4 : 3;
@@ -398,6 +401,7 @@ __global__ void __launch_bounds__(L / E) k_born1d(Born1DArgs a)
 template <class T, int N2, int E, int W>
 __global__ void __launch_bounds__(W *(N2 / E)) k_born_fs_col(BornFsColArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TM = Plan<N2, E>::TL;
     constexpr int NT = W * TM;
@@ -491,6 +495,7 @@ __global__ void __launch_bounds__(W *(N2 / E)) k_born_fs_col(BornFsColArgs a)
 template <class T, int N1, int E, int B>
 __global__ void __launch_bounds__(B *(N1 / E)) k_born_fs_row(BornFsRowArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = Plan<N1, E>::TL;
     constexpr int PADS = sizeof(C) == 8 ? 4 : 3;

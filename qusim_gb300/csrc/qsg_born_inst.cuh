@@ -51,7 +51,7 @@ static cudaError_t run_born_row(int nx, const BornRowArgs &a, cudaStream_t st)
     auto k = k_born_row<T, NY, E, G, B>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<nx / (G * B), B * G * (NY / E), smem, st>>>(a);
+    launch_pdl(k, dim3(nx / (G * B)), dim3(B * G * (NY / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -63,7 +63,7 @@ static cudaError_t run_born_col(int ny, int g, const BornColArgs &a, cudaStream_
     auto k = k_born_col<T, M, E, W>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<g * (ny / W), W * (M / E), smem, st>>>(a);
+    launch_pdl(k, dim3(g * (ny / W)), dim3(W * (M / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -76,7 +76,7 @@ static cudaError_t run_born_1d(const Born1DArgs &a, cudaStream_t st)
     auto k = k_born1d<T, L, E>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<1, L / E, smem, st>>>(a);
+    launch_pdl(k, dim3(1), dim3(L / E), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -88,7 +88,7 @@ static cudaError_t run_born_fs_col(int n1, const BornFsColArgs &a, cudaStream_t 
     auto k = k_born_fs_col<T, N2, E, W>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<n1 / W, W * (N2 / E), smem, st>>>(a);
+    launch_pdl(k, dim3(n1 / W), dim3(W * (N2 / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -101,7 +101,7 @@ static cudaError_t run_born_fs_row(int n2, const BornFsRowArgs &a, cudaStream_t 
     auto k = k_born_fs_row<T, N1, E, B>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<n2 / B, B * (N1 / E), smem, st>>>(a);
+    launch_pdl(k, dim3(n2 / B), dim3(B * (N1 / E)), smem, st, a);
     return cudaGetLastError();
 }
 

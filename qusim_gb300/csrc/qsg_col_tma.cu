@@ -26,7 +26,7 @@ static cudaError_t run_col_tma(const ColPassArgs &a, const CUtensorMap *mw, cons
     }
     // persistent: one CTA per SM (the staging buffers take most of its shared memory)
     const int grid = std::min(a.tiles, sm_count());
-    k<<<grid, W * (M / E), smem, st>>>(a, *mw, *mp);
+    launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a, *mw, *mp);
     return cudaGetLastError();
 }
 

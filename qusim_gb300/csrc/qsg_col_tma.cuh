@@ -98,6 +98,7 @@ template <int M, int E, int W, bool PL>
 __global__ void __launch_bounds__(W *(M / E), 1)
     k_col_pass_tma(ColPassArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_p)
 {
+    pdl_wait();
     using C = float2;
     using TW = pass_tw_t<C, PL>;
     using P = Plan<M, E>;

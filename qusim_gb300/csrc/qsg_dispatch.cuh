@@ -15,6 +15,28 @@ static inline cudaError_t prepare_smem(K kernel, size_t smem)
     return cudaSuccess;
 }
 
+// Launch a kernel that starts with pdl_wait() as a programmatic dependent of the
+// kernel before it on the stream.  The wait keeps the order and the visibility of
+// a plain launch; what goes away is the gap between the two: back-to-back plain
+// launches cost 2 to 4 us on this part, rounded up to steps of 2.05 us (measured
+// with kernels of 0 .. 8 us: 4.1, 4.1, 6.15, 8.2 us a launch for 0, 1, 2, 4 us of
+// work), dependent ones 0.9 us over the work (1.4, 1.9, 2.9, 4.95 us).
+template <class... P, class... A>
+static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Multiprocessors of the current device (cached per device).
 static inline int sm_count()
 {

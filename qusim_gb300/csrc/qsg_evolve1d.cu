@@ -25,7 +25,7 @@ static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
     auto k = k_evolve1d_resident<T, L, E, NI, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(a.count + NI - 1) / NI, NI * (L / E), smem, st>>>(a);
+    launch_pdl(k, dim3((a.count + NI - 1) / NI), dim3(NI * (L / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -57,7 +57,7 @@ static cudaError_t run_queue(const Evolve1DQueueArgs &a, cudaStream_t st)
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     static int occ = 0;
-    k<<<persistent_grid(k, QT / E, smem, a.ntiles, occ), QT / E, smem, st>>>(a);
+    launch_pdl(k, dim3(persistent_grid(k, QT / E, smem, a.ntiles, occ)), dim3(QT / E), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -118,7 +118,7 @@ static cudaError_t run_wall(const Evolve1DBatchArgs &a, cudaStream_t st)
     auto k = k_evolve1d_wall<T, L2, E, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<a.count, L2 / E, smem, st>>>(a);
+    launch_pdl(k, dim3(a.count), dim3(L2 / E), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -219,7 +219,7 @@ static cudaError_t run_fs_col(const FsGeom &g, const FsColArgs &a, int ninst, cu
     auto k = k_fs_col<T, N2, E, W, FX>;
     cudaError_t e = prepare_smem(k, g.col_smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(g.col_blocks, ninst), W * (N2 / E), g.col_smem, st>>>(a);
+    launch_pdl(k, dim3(g.col_blocks, ninst), dim3(W * (N2 / E)), g.col_smem, st, a);
     return cudaGetLastError();
 }
 
@@ -235,7 +235,7 @@ static cudaError_t run_fs_row(const FsGeom &g, const FsRowArgs &a, int ninst, cu
     auto k = k_fs_row<T, N1, E, B, FX>;
     cudaError_t e = prepare_smem(k, g.row_smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(g.row_blocks, ninst), B * (N1 / E), g.row_smem, st>>>(a);
+    launch_pdl(k, dim3(g.row_blocks, ninst), dim3(B * (N1 / E)), g.row_smem, st, a);
     return cudaGetLastError();
 }
 

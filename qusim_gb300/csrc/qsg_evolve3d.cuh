@@ -60,6 +60,7 @@ constexpr int min_blocks3(int threads) { return threads <= 256 ? 3 : 1; }
 template <class T, int L, int E, int B>
 __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = Plan<L, E>::TL;
     constexpr int NT = B * TL;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
 template <class T, int L, int E, int W>
 __global__ void __launch_bounds__(W *(L / E), min_blocks3(W *(L / E))) k3_col(Pass3Args a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TM = Plan<L, E>::TL;
     constexpr int NT = W * TM;

@@ -21,7 +21,7 @@ static cudaError_t run3_row(size_t lines, const Pass3Args &a, cudaStream_t st)
     auto k = k3_row<T, L, E, B>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)(lines / B), B * (L / E), smem, st>>>(a);
+    launch_pdl(k, dim3((unsigned)(lines / B)), dim3(B * (L / E)), smem, st, a);
     return cudaGetLastError();
 }
 
@@ -33,7 +33,7 @@ static cudaError_t run3_col(int inner, int outer, const Pass3Args &a, cudaStream
     auto k = k3_col<T, L, E, W>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(inner / W, outer), W * (L / E), smem, st>>>(a);
+    launch_pdl(k, dim3(inner / W, outer), dim3(W * (L / E)), smem, st, a);
     return cudaGetLastError();
 }
 

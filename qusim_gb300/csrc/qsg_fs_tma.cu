@@ -26,7 +26,7 @@ static cudaError_t run_fs_tma(const FsColArgs &a, cudaStream_t st)
     }
     static int occ = 0;
     const unsigned grid = persistent_grid(k, W * (N2 / 16), smem, a.tiles, occ);
-    k<<<grid, W * (N2 / 16), smem, st>>>(a);
+    launch_pdl(k, dim3(grid), dim3(W * (N2 / 16)), smem, st, a);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@ __host__ __device__ constexpr size_t fs_tma_smem(int n2, int w) { return fs_tma_
 template <int N2, int W>
 __global__ void __launch_bounds__(W *(N2 / 16), 2) k_fs_col_tma(FsColArgs a)
 {
+    pdl_wait();
     using C = float2;
     constexpr int E = 16;
     constexpr int TM = Plan<N2, E>::TL;

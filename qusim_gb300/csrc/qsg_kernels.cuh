@@ -57,6 +57,9 @@ template <> struct PhaseOps<float2> {
 };
 
 template <class C> __device__ __forceinline__ C ld_c(const C *p) { return __ldg(p); }
+// First statement of every kernel that is launched with launch_pdl: waits for
+// the kernels before it on the stream and their writes (see launch_pdl).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Streaming loads of psi and of the V tables bypass L1: each element is read
 // once per pass, and letting them allocate evicts the twiddle tables that
 // every butterfly stage re-reads from L1.
@@ -437,6 +440,7 @@ template <class T, int NY, int E, int G, int B, int RS, bool PL = false, bool FX
 __global__ void __launch_bounds__(B *G *(NY / E) / RS, sizeof(T) == 8 ? (G == 1 ? 768 : 512) / (B * G * (NY / E) / RS) : 0)
     k_row_pass(RowPassArgs a)
 {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[32];
     if (a.in_split)
@@ -477,6 +481,7 @@ template <class T, int M, int E, int W, bool PL = false, bool FX = false>
 __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : sizeof(T) == 8 ? 1024 / (W * (M / E)) : 1)
     k_col_pass(ColPassArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     using TW = pass_stw_t<C, PL>;
     using P = Plan<M, E>;
@@ -754,6 +759,7 @@ template <class T, int N2, int E, int W, bool FX = false>
 __global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T) == 4 || FX) ? 768 / (W * (N2 / E)) : 1)
     k_fs_col(FsColArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TM = Plan<N2, E>::TL;
     constexpr int NT = W * TM;
@@ -893,6 +899,7 @@ template <class T, int N1, int E, int B, bool FX = false>
 __global__ void __launch_bounds__(B *(N1 / E), FX && B * (N1 / E) <= 256 ? 768 / (B * (N1 / E)) : 0)
     k_fs_row(FsRowArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = Plan<N1, E>::TL;
     constexpr int PADS = sizeof(C) == 8 ? 4 : 3;
@@ -1140,6 +1147,7 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
 template <class T, int L, int E, int NI, bool FX>
 __global__ void __launch_bounds__(NI *(L / E)) k_evolve1d_resident(Evolve1DBatchArgs a)
 {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     const int first = blockIdx.x * NI;
     evolve1d_lines<T, L, E, NI, FX>(a, first, a.count - first, a.tw, smraw);
@@ -1170,6 +1178,7 @@ struct Evolve1DQueueArgs {
 template <class T, int QT, int E>
 __global__ void __launch_bounds__(QT / E) k_evolve1d_queue(Evolve1DQueueArgs a)
 {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int tile_s;
 #pragma unroll 1
@@ -1232,6 +1241,7 @@ __device__ __forceinline__ void odd_extend(C (&x)[E], C *sm, const Lay &lay, int
 template <class T, int L2, int E, bool FX = false>
 __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
 {
+    pdl_wait();
     using C = cplx_t<T>;
     constexpr int TL = L2 / E;
     constexpr int H = E / 2;  // slots holding psi

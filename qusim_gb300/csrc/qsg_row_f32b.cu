@@ -18,7 +18,7 @@ static cudaError_t run_row_f32b(const Geom2D &g, const RowPassArgs &a, cudaStrea
     cudaError_t e = prepare_smem(k, g.row_smem);
     if (e != cudaSuccess) return e;
     static int occ = 0;
-    k<<<persistent_grid(k, NT, g.row_smem, a.units, occ), NT, g.row_smem, st>>>(a);
+    launch_pdl(k, dim3(persistent_grid(k, NT, g.row_smem, a.units, occ)), dim3(NT), g.row_smem, st, a);
     return cudaGetLastError();
 }
 

@@ -29,7 +29,7 @@ static cudaError_t run_row_tm(const RowPassArgs &a, cudaStream_t st)
     // one CTA per SM: each takes all 512 TMEM columns of its SM
     const int ctas = (a.units + NG - 1) / NG;
     const int sms = sm_count();
-    k<<<(unsigned)(ctas < sms ? ctas : sms), 512, smem, st>>>(a);
+    launch_pdl(k, dim3((unsigned)(ctas < sms ? ctas : sms)), dim3(512), smem, st, a);
     return cudaGetLastError();
 }
 

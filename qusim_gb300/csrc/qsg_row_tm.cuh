@@ -260,6 +260,7 @@ __device__ __forceinline__ void row_tm_units(const RowPassArgs &a, float2 *sm, d
 template <int NY, bool PL = false>
 __global__ void __launch_bounds__(512, 1) k_row_pass_tm(RowPassArgs a)
 {
+    pdl_wait();
     constexpr int NT = NY / 16;
     constexpr int LINE = padded<NY, 4>(NY);
     extern __shared__ __align__(16) unsigned char smraw[];
