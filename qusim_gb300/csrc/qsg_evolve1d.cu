@@ -1,5 +1,5 @@
 // 1D evolution: batched resident kernel, four-step passes, kinetic transforms.
-#include "qsg_dispatch.cuh"
+#include "qsg_evolve1d_inst.cuh"
 
 namespace qsg {
 
@@ -10,25 +10,6 @@ bool evolve1d_supported(int prec, uint64_t n)
     if (n < 64 || (n & (n - 1))) return false;
     return prec == 1 ? n <= 8192 : n <= 4096;
 }
-constexpr int res_ni_for(int l, int e) { return (256 / (l / e)) > 1 ? 256 / (l / e) : 1; }
-
-template <class T, int L, bool FX = false>
-static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_evolve1d<T, L, true>(a, st);
-    }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
-    constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
-    constexpr int NI = res_ni_for(L, E);
-    const size_t smem = sizeof(cplx_t<T>) * padded<L, PADS>(L) * NI;
-    auto k = k_evolve1d_resident<T, L, E, NI, FX>;
-    cudaError_t e = prepare_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3((a.count + NI - 1) / NI), dim3(NI * (L / E)), smem, st, a);
-    return cudaGetLastError();
-}
-
 template <class T, int L>
 static cudaError_t run_kinetic1d(const void *psi, const void *tw, double dtk, double *sums,
                                  cudaStream_t st)
@@ -68,18 +49,21 @@ cudaError_t launch_evolve1d_queue(int prec, const Evolve1DQueueArgs &a, cudaStre
     return run_queue<float, 8192>(a, st);
 }
 
-#define QSG_1D_CASES(X, T) \
-    X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048) X(T, 4096)
-
 cudaError_t launch_evolve1d(int prec, int n, const Evolve1DBatchArgs &a, cudaStream_t st)
 {
-#define X(T, L) case L: return run_evolve1d<T, L>(a, st);
+    const bool few = n >= 64 && res_few(n, prec == 1 ? 16 : 8, a.count);
+    if (prec == 1 && few) return launch_evolve1d_few_f32(n, a, st);
+#define X(T, L) case L: return run_evolve1d<T, L, false>(a, st);
+#define Y(T, L) case L: return run_evolve1d<T, L, true>(a, st);
     if (prec == 1) {
         switch (n) { QSG_1D_CASES(X, float) X(float, 8192) default: break; }
+    } else if (few) {
+        switch (n) { QSG_1D_CASES(Y, double) default: break; }
     } else {
         switch (n) { QSG_1D_CASES(X, double) default: break; }
     }
 #undef X
+#undef Y
     return cudaErrorNotSupported;
 }
 
@@ -106,22 +90,6 @@ bool wall1d_supported(int prec, uint64_t n)
     return prec == 1 ? 2 * n <= 8192 : 2 * n <= 4096;
 }
 
-template <class T, int L2, bool FX = false>
-static cudaError_t run_wall(const Evolve1DBatchArgs &a, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_wall<T, L2, true>(a, st);
-    }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
-    constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
-    const size_t smem = sizeof(cplx_t<T>) * padded<L2, PADS>(L2);
-    auto k = k_evolve1d_wall<T, L2, E, FX>;
-    cudaError_t e = prepare_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3(a.count), dim3(L2 / E), smem, st, a);
-    return cudaGetLastError();
-}
-
 template <class T, int L2>
 static cudaError_t run_wallkin(const void *psi, const void *tw, double dtk, double *sums, cudaStream_t st)
 {
@@ -137,12 +105,9 @@ static cudaError_t run_wallkin(const void *psi, const void *tw, double dtk, doub
 
 cudaError_t launch_wall1d(int prec, int n, const Evolve1DBatchArgs &a, cudaStream_t st)
 {
+    if (prec == 1) return launch_wall1d_f32(n, a, st);
 #define X(T, L) case L / 2: return run_wall<T, L>(a, st);
-    if (prec == 1) {
-        switch (n) { QSG_1D_CASES(X, float) X(float, 8192) default: break; }
-    } else {
-        switch (n) { QSG_1D_CASES(X, double) default: break; }
-    }
+    switch (n) { QSG_1D_CASES(X, double) default: break; }
 #undef X
     return cudaErrorNotSupported;
 }
