@@ -1843,10 +1843,12 @@ namespace {
 // complex): ext_j = psi_j (j < n), 0 at j = n, ext_{2n-j} = -psi_j (0 < j < n).
 // Site 0 keeps psi_0 as given: the reference discards it (and site n) only when
 // a kinetic factor is applied; step1d zeroes it before the first step.
-int wall_odd_extension(const double *psi, uint64_t n, std::vector<double> &ext)
+int wall_odd_extension(qsg_ctx *ctx, const double *psi, uint64_t n, std::vector<double> &ext)
 {
     std::vector<double> h(2 * n);
-    QSG_CUDA(cudaMemcpy(h.data(), psi, sizeof(double) * 2 * n, cudaMemcpyDefault));
+    // (a device source may still be being sampled on the context's stream)
+    QSG_CUDA(cudaMemcpyAsync(h.data(), psi, sizeof(double) * 2 * n, cudaMemcpyDefault, ctx->st));
+    QSG_CUDA(cudaStreamSynchronize(ctx->st));
     ext.assign(4 * n, 0.0);
     std::memcpy(ext.data(), h.data(), sizeof(double) * 2 * n);
     for (uint64_t j = 1; j < n; ++j) {
@@ -1857,10 +1859,11 @@ int wall_odd_extension(const double *psi, uint64_t n, std::vector<double> &ext)
 }
 
 // V on the extension: even (V_{2n-j} = V_j), 0 at j = n (where the state is 0)
-int wall_even_extension(const double *V, uint64_t n, std::vector<double> &ext)
+int wall_even_extension(qsg_ctx *ctx, const double *V, uint64_t n, std::vector<double> &ext)
 {
     std::vector<double> h(n);
-    QSG_CUDA(cudaMemcpy(h.data(), V, sizeof(double) * n, cudaMemcpyDefault));
+    QSG_CUDA(cudaMemcpyAsync(h.data(), V, sizeof(double) * n, cudaMemcpyDefault, ctx->st));
+    QSG_CUDA(cudaStreamSynchronize(ctx->st));
     ext.assign(2 * n, 0.0);
     std::memcpy(ext.data(), h.data(), sizeof(double) * n);
     for (uint64_t j = 1; j < n; ++j) ext[2 * n - j] = h[j];
@@ -1970,8 +1973,8 @@ static int create_1d_locked(qsg_ctx *ctx, uint64_t n, double dx, double mass, do
     }
     if (!rc && wall_ext) {
         std::vector<double> pe, ve;
-        rc = wall_odd_extension(psi0, n, pe);
-        if (!rc) rc = wall_even_extension(V, n, ve);
+        rc = wall_odd_extension(ctx, psi0, n, pe);
+        if (!rc) rc = wall_even_extension(ctx, V, n, ve);
         if (!rc) rc = common_create(in, pe.data(), ve.data());
     } else if (!rc) {
         rc = common_create(in, psi0, V);
@@ -2656,7 +2659,7 @@ int qsg_set_psi(qsg_inst *in, const double *psi)
     int rc;
     if (in->wall_ext) {
         std::vector<double> pe;
-        if ((rc = wall_odd_extension(psi, in->n_out, pe))) return rc;
+        if ((rc = wall_odd_extension(in->ctx, psi, in->n_out, pe))) return rc;
         rc = upload_psi(in, pe.data());
         if (!rc) QSG_CUDA(cudaStreamSynchronize(in->ctx->st));  // pe is pageable and goes out of scope
     } else {
