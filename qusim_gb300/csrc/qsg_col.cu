@@ -169,8 +169,20 @@ bool default_plan(int prec, int nx, int ny, Plan2D *p)
             c.col_e = 32;
             c.col_w = 16;
         }
+        // Small grids leave lanes idle and are bound by the instructions one
+        // thread runs in a row: radix 8 (twice the threads), shorter columns, fewer
+        // columns per CTA.  Per O4 step against the rule above: 128^2 16.5 / 23.5
+        // us, 256^2 17.5 / 24.0, 512^2 22.3 / 36.4, 1024 x 512 34.2 / 38.4; 1024^2
+        // and 128 x 4096 no longer gain.  (Errors over 200 steps agree within 3%.)
+        const long sites = (long)nx * ny;
+        if (sites <= 262144 || (sites <= 524288 && nx >= 1024)) {
+            c.g = nx >= 512 ? 4 : 1;
+            c.row_e = c.col_e = 8;
+            c.row_nt = 256;
+            c.col_w = nx / c.g == 128 ? 8 : (nx == 256 ? 4 : (nx / c.g == 256 ? 8 : 4));
+        }
         // rows of 2048 / 4096 points in 4-row units: waiting rows parked in TMEM
-        if (c.g == 4 && row_tm_supported(ny, c.g)) {
+        if (c.g == 4 && c.row_e == 16 && row_tm_supported(ny, c.g)) {
             c.row_nt = 512;
             c.row_kind = 1;
         }
@@ -191,7 +203,7 @@ bool default_plan(int prec, int nx, int ny, Plan2D *p)
         const int tl = ny / c.row_e;
         c.row_nt = c.g > 1 ? (row_work_for(ny, 8, c.g, 256) >= 512 ? 512 : 256) : small ? 128 : (tl > 64 ? tl : 64);
         c.col_e = small ? 4 : 8;
-        c.col_w = small || m >= 1024 ? 2 : 4;
+        c.col_w = small || m >= 1024 || (m == 512 && (long)nx * ny > 262144) ? 2 : 4;
     }
     Geom2D g;
     if (geom2d(prec, nx, ny, c, &g)) {
