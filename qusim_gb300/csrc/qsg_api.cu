@@ -700,31 +700,42 @@ int step2d(qsg_inst *in, uint64_t nsteps, int renorm)
     return QSG_OK;
 }
 
-// 3D: one pass over the lines of an axis (0 x, 1 y, 2 z): [vpre] F^-1 K F [vpost]
-template <class T>
-int pass3(qsg_inst *in, int ax, int ktab, const void *vpre, bool pre2, const void *vpost, bool post2, double *kin)
+// One 3D pass over the lines of an axis (0 x, 1 y, 2 z) of the planes
+// [x0, x0 + planes) of the first axis (all of them for axis 0):
+// [v0] F^-1 K F [v1] [F^-1 K' F] [v2]; kt, kt2: kinetic tables (kt2 < 0: none)
+struct Pass3 {
+    int ax, kt, kt2 = -1;
+    const void *v0 = nullptr, *v1 = nullptr, *v2 = nullptr;
+    bool twice = false;  // v1 applied twice
+};
+template <class T> int pass3(qsg_inst *in, const Pass3 &p, int x0, int planes, double *kin = nullptr)
 {
     qsg::Pass3Args a{};
-    a.psi = in->psi;
-    a.vpre = vpre;
-    a.vpre_twice = pre2 ? 1 : 0;
-    a.vpost = vpost;
-    a.vpost_twice = post2 ? 1 : 0;
-    a.k = in->k3[ax][ktab];
-    a.tw = in->tw3[ax];
+    const int nx = in->nx, ny = in->ny, nz = in->nz;
+    const size_t off = (size_t)x0 * ny * nz * csize(in->prec);
+    auto at = [&](const void *q) { return q ? static_cast<const char *>(q) + off : nullptr; };
+    a.psi = static_cast<char *>(in->psi) + off;
+    a.v[0] = at(p.v0);
+    a.v[1] = at(p.v1);
+    a.v[2] = at(p.v2);
+    a.vmid_twice = p.twice ? 1 : 0;
+    a.k = in->k3[p.ax][p.kt];
+    a.k2 = p.kt2 >= 0 ? in->k3[p.ax][p.kt2] : nullptr;
+    a.fx = in->fx ? 1 : 0;
+    a.n = in->n - (size_t)x0 * ny * nz;
+    a.tw = in->tw3[p.ax];
     a.partials = kin;
     a.kinetic = kin ? 1 : 0;
-    const int nx = in->nx, ny = in->ny, nz = in->nz;
     const int L[3] = {nx, ny, nz};
-    a.inv_l = (float)(1.0 / L[ax]);
-    if (ax == 2) {
+    a.inv_l = (float)(1.0 / L[p.ax]);
+    if (p.ax == 2) {
         ProfScope ps(in->ctx, "pass3_z", in->st);
-        QSG_CUDA(qsg::launch3_row<T>(nz, (size_t)nx * ny, a, in->st));
-    } else if (ax == 1) {
+        QSG_CUDA(qsg::launch3_row<T>(nz, (size_t)planes * ny, a, in->st));
+    } else if (p.ax == 1) {
         a.s_line = nz;
         a.s_outer = (long long)ny * nz;
         ProfScope ps(in->ctx, "pass3_y", in->st);
-        QSG_CUDA(qsg::launch3_col<T>(ny, nz, nx, a, in->st));
+        QSG_CUDA(qsg::launch3_col<T>(ny, nz, planes, a, in->st));
     } else {
         a.s_line = (long long)ny * nz;
         a.s_outer = nz;
@@ -734,37 +745,34 @@ int pass3(qsg_inst *in, int ax, int ktab, const void *vpre, bool pre2, const voi
     return QSG_OK;
 }
 
-// O2: z[V V', Kz] y[Ky] x[Kx, (V)];  O4: z[V1 V1', K1] y x[V2] z[K2] y x[V2] z[K1] y x[(V1)]
-template <class T> int step3d_t(qsg_inst *in, uint64_t nsteps, int renorm)
+// The passes of a call (qsg_evolve3d.cuh): z[V, K] y x[K, V, K] y z[K, V, K] y ... [K, V].
+template <class T> int step3d_t(qsg_inst *in, uint64_t nsteps)
 {
-    int rc;
     const void *V0 = in->vtab[0], *V1 = in->vtab[1];
-    for (uint64_t s = 0; s < nsteps; ++s) {
-        const bool last = s + 1 == nsteps;
-        const void *close = last ? V0 : nullptr;
-        if (in->order == 2) {
-            if ((rc = pass3<T>(in, 2, 0, V0, s > 0, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 1, 0, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 0, 0, nullptr, false, close, false, nullptr))) return rc;
-        } else {
-            if ((rc = pass3<T>(in, 2, 0, V0, s > 0, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 1, 0, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 0, 0, nullptr, false, V1, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 2, 1, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 1, 1, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 0, 1, nullptr, false, V1, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 2, 0, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 1, 0, nullptr, false, nullptr, false, nullptr))) return rc;
-            if ((rc = pass3<T>(in, 0, 0, nullptr, false, close, false, nullptr))) return rc;
+    const uint64_t nsub = in->order == 2 ? 1 : 3, subs = nsteps * nsub;
+    auto kt = [&](uint64_t i) { return in->order == 4 && i % 3 == 1 ? 1 : 0; };  // O4: K1 K2 K1
+    if (subs == 0) return QSG_OK;
+    int rc;
+    Pass3 first{2, kt(0)};
+    first.v0 = V0;
+    if ((rc = pass3<T>(in, first, 0, in->nx))) return rc;
+    for (uint64_t i = 0; i < subs; ++i) {
+        if ((rc = pass3<T>(in, Pass3{1, kt(i)}, 0, in->nx))) return rc;
+        Pass3 p{i % 2 == 0 ? 0 : 2, kt(i)};
+        const bool join = i % nsub == nsub - 1;  // the step's last substep
+        p.v1 = in->order == 4 && !join ? V1 : V0;
+        if (i + 1 < subs) {
+            p.kt2 = kt(i + 1);
+            p.twice = join;  // the step's closing factor and the next one's opening factor
         }
+        if ((rc = pass3<T>(in, p, 0, in->nx))) return rc;
     }
-    (void)renorm;
     return QSG_OK;
 }
 
 int step3d(qsg_inst *in, uint64_t nsteps, int renorm)
 {
-    int rc = in->prec == 1 ? step3d_t<float>(in, nsteps, renorm) : step3d_t<double>(in, nsteps, renorm);
+    int rc = in->prec == 1 ? step3d_t<float>(in, nsteps) : step3d_t<double>(in, nsteps);
     if (rc || !renorm) return rc;
     // renormalise at the end of the call, as 2D does (QuEvolverImpl::Step, src/EvolverImpl.cpp:56-68)
     qsg_ctx *ctx = in->ctx;
@@ -786,8 +794,8 @@ int kinetic3d(qsg_inst *in, double *kin)
     for (int ax = 0; ax < 3; ++ax) {
         const int ctas = ax == 2 ? qsg::row3_ctas(in->prec, in->nz, (size_t)in->nx * in->ny)
                                  : qsg::col3_ctas(in->prec, L[ax], in->nz, ax == 1 ? in->nx : in->ny);
-        int rc = in->prec == 1 ? pass3<float>(in, ax, 0, nullptr, false, nullptr, false, in->kparts3)
-                               : pass3<double>(in, ax, 0, nullptr, false, nullptr, false, in->kparts3);
+        int rc = in->prec == 1 ? pass3<float>(in, Pass3{ax, 0}, 0, in->nx, in->kparts3)
+                               : pass3<double>(in, Pass3{ax, 0}, 0, in->nx, in->kparts3);
         if (rc) return rc;
         std::vector<double> h(2 * (size_t)ctas);
         QSG_CUDA(cudaMemcpyAsync(h.data(), in->kparts3, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->st));
@@ -1353,7 +1361,7 @@ int build_tables(qsg_inst *in)
             for (int k = 0; k < ntab; ++k) {
                 const cd f = alpha * tc[k] * DT;
                 if ((rc = inst_alloc(in, (size_t)L[ax] * cs, &in->k3[ax][k]))) return rc;
-                QSG_CUDA(qsg::launch_ktable1d(in->prec, in->k3[ax][k], L[ax], f.real(), f.imag(),
+                QSG_CUDA(qsg::launch_ktable1d(tab_prec(in), in->k3[ax][k], L[ax], f.real(), f.imag(),
                                               1.0 / (double)L[ax], ctx->st));
             }
         }
@@ -2277,6 +2285,11 @@ int qsg_create_3d(qsg_ctx *ctx, uint64_t nx, uint64_t ny, uint64_t nz, double dx
     in->order = order;
     in->prec = precision;
     in->st = ctx->st;
+    {
+        const double kx = kPi / dx * hbar, ky = kPi / dy * hbar, kz = kPi / dz * hbar;
+        in->fx = precision == 0 && dt_im == 0 &&
+                 std::isfinite((kx * kx + ky * ky + kz * kz) / (2 * mass) * dt_re * 2 / hbar);
+    }
     int rc = common_create(in, psi0, V);
     if (rc) {
         std::string msg = g_last_error;

@@ -6,19 +6,21 @@
 // evolver; this is SplittingMethod2D's step (src/SplittingMethod2D.cpp:38-121)
 // with a third axis.  The kinetic factor exp(a (kx^2 DTx + ky^2 DTy + kz^2 DTz))
 // is a product of one factor per axis, so the kinetic operator is the product
-// of three commuting one-axis operators F_a^-1 K_a F_a: each is one pass over
-// the lines along its axis (transform, factor, inverse transform, all on chip),
-// and V multiplies fuse into the passes.  A step never leaves natural
-// real-space layout:
+// of three commuting one-axis operators F_a^-1 K_a F_a: each is a pass over the
+// lines along its axis (transform, factor, inverse transform, all on chip), and
+// V multiplies fuse into the passes.  A step never leaves natural real-space
+// layout.  Because the axes commute, a kinetic substep may take them in either
+// order: substeps alternate z y x and x y z, and the last axis of one, the V
+// between and the same axis of the next are one pass of four transforms.  With
+// s substeps in a call (1 per step in O2, 3 in O4) that is 2 s + 1 passes:
 //
-//   O2: z[V V', Kz] y[Ky] x[Kx, (V)]                   3 passes
-//   O4: z[V1 V1', Kz1] y[Ky1] x[Kx1, V2] z[Kz2] y[Ky2] x[Kx2, V2]
-//       z[Kz1] y[Ky1] x[Kx1, (V1)]                     9 passes
+//   z[V, Kz] y[Ky] x[Kx, V, Kx] y[Ky] z[Kz, V, Kz] y[Ky] x[Kx, V, Kx] ... [K, V]
 //
-// (V' = the previous step's closing factor, merged; (V) only on the last step
-// of a call.)  z lines are contiguous (k3_row); y and x lines are strided by nz
-// and ny*nz (k3_col, W adjacent z positions per CTA so every access is a W-wide
-// contiguous segment).
+// against 3 s of one axis each (O4 per step: 256^3 complex64 747 -> 602 us,
+// complex128 with the products in fixed point as well 16.5 -> 3.61 ms).
+// z lines are contiguous (k3_row); y and x lines are strided by nz and ny*nz
+// (k3_col, W adjacent z positions per CTA so every access is a W-wide contiguous
+// segment).
 #pragma once
 #include "qsg_kernels.cuh"
 
@@ -26,10 +28,13 @@ namespace qsg {
 
 struct Pass3Args {
     void *psi;
-    const void *vpre;      // V factor before the line transforms (or null) ...
-    const void *vpost;     // ... and after (or null); natural layout, n entries
-    int vpre_twice, vpost_twice;
-    const void *k;         // the axis factor: complex64 factor - 1, complex128 factor / L
+    const void *v[3];      // V factor before the axis operator, after it (before a second one),
+                           // after the second (or null each); natural layout, n entries
+    int vmid_twice;        // v[1] applied twice (the two ExpV calls at a step boundary)
+    const void *k, *k2;    // the axis factor, and a second one (or null): complex64 factor - 1,
+                           // complex128 factor / L (FX: fixed-point factors)
+    int fx;
+    size_t n;              // sites (FX: the V tables' flag entry)
     const void *tw;        // stage twiddles (L, E)
     float inv_l;           // 1/L (complex64)
     long long s_line;      // stride between a line's elements (strided kernel)
@@ -38,11 +43,15 @@ struct Pass3Args {
     int kinetic;           // 1: forward transform and the kinetic sums only (no store)
 };
 
-template <class C> __device__ __forceinline__ C v3_apply(C x, const C *vt, size_t i, int twice)
+template <class C, int E, class I> __device__ __forceinline__ void v3_apply(C (&x)[E], const void *v, I idx, bool twice)
 {
-    const C v = ld_stream(vt + i);
-    x = PhaseOps<C>::apply(x, v);
-    return twice ? PhaseOps<C>::apply(x, v) : x;
+    const C *vt = opaque(static_cast<const C *>(v));
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const C m = ld_stream(vt + idx(e));
+        x[e] = PhaseOps<C>::apply(x[e], m);
+        if (twice) x[e] = PhaseOps<C>::apply(x[e], m);
+    }
 }
 
 // x * K[k] (with 1/L): complex64 cmul1p on the factor - 1 table
@@ -52,13 +61,73 @@ template <class C> __device__ __forceinline__ C k3_apply(C x, const C *kt, int k
     else return cmul(x, ld_c(kt + k));
 }
 
+// [V] F^-1 K F [V] [F^-1 K2 F] [V] on a line in registers, the inverse as
+// conj(F(conj(.))); idx(e): the site of slot e.  One transform body in a loop.
+// FX (complex128, real time steps): the line is in fixed point throughout.
+template <class C, int L, int E, bool FX, class Lay, class Bar, class I>
+__device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const Bar &bar, int t, const stw_t<C> *tw,
+                                         const Pass3Args &a, I idx)
+{
+    constexpr int TL = L / E;
+    const int nq = a.k2 ? 4 : 2;
+    if constexpr (FX) {
+        FixLine<L, E> f;
+        f.load(x, sm, lay, bar, t);
+        auto mul_v = [&](const void *v, bool twice) {
+            const fixw *vt = opaque(static_cast<const fixw *>(v));
+            if (fix_flagged(vt + a.n)) f.finite = false;
+            f.mul([&](int e) { return ld_stream(vt + idx(e)); }, twice);
+        };
+        if (a.v[0]) mul_v(a.v[0], false);
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q) {
+            f.fft(sm, lay, bar, t, opaque(tw));
+            f.scale(sm, lay, bar, t);
+            if ((q & 1) == 0) {
+                const fixw *kt = static_cast<const fixw *>(q ? a.k2 : a.k);
+                f.ex -= Plan<L, E>::LOGL;  // 1/L
+                f.mul([&](int e) { return __ldg(kt + t + e * TL); }, false);
+                f.conj();
+            } else {
+                f.conj();
+                const void *v = q == 1 ? a.v[1] : a.v[2];
+                if (v)
+                    mul_v(v, q == 1 && a.vmid_twice);
+                else if (q + 1 < nq)
+                    f.quarter();
+            }
+        }
+        f.store(x);
+    } else {
+        if (a.v[0]) v3_apply(x, a.v[0], idx, false);
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q) {
+            line_fft<C, L, E, false>(x, sm, lay, bar, t, tw);
+            if ((q & 1) == 0) {
+                const C *kt = static_cast<const C *>(q ? a.k2 : a.k);
+#pragma unroll
+                for (int e = 0; e < E; ++e) x[e] = cconj(k3_apply(x[e], kt, t + e * TL, a.inv_l));
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
+                const void *v = q == 1 ? a.v[1] : a.v[2];
+                if (v) v3_apply(x, v, idx, q == 1 && a.vmid_twice);
+            }
+        }
+    }
+}
+
 // B contiguous lines (z) of L per CTA
 // strided passes: three 256-thread CTAs per SM (registers capped at 85), as
 // they are bound by the latency of their scattered loads, not by issue
 constexpr int min_blocks3(int threads) { return threads <= 256 ? 3 : 1; }
+// contiguous lines: the same, except lines within a warp, whose loads the
+// compiler schedules across __syncwarp: at 85 registers they spill 270 bytes (z
+// of 256^3 150 us a pass of four transforms, 131 with two CTAs per SM)
+constexpr int min_blocks3_row(int threads, int tl) { return threads > 256 ? 1 : (tl <= 32 ? 2 : 3); }
 
-template <class T, int L, int E, int B>
-__global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
+template <class T, int L, int E, int B, bool FX = false>
+__global__ void __launch_bounds__(B *(L / E), min_blocks3_row(B *(L / E), L / E)) k3_row(Pass3Args a)
 {
     pdl_wait();
     using C = cplx_t<T>;
@@ -76,7 +145,6 @@ __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
     const auto lbar = LineBarrierOf<TL, B>::make(line);
     C *psi = static_cast<C *>(a.psi);
     const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
-    const C *kt = static_cast<const C *>(a.k);
 
     C x[E];
 #pragma unroll
@@ -100,26 +168,7 @@ __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
         }
         return;
     }
-    if (a.vpre) {
-        const C *vt = opaque(static_cast<const C *>(a.vpre));
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = v3_apply(x[e], vt, base + e * TL, a.vpre_twice);
-    }
-    // F^-1 K F, the inverse as conj(F(conj(.)))
-#pragma unroll 1
-    for (int q = 0; q < 2; ++q) {
-        line_fft<C, L, E, false>(x, sm, lay, lbar, t, tw);
-        if (q == 1) continue;
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = cconj(k3_apply(x[e], kt, t + e * TL, a.inv_l));
-    }
-#pragma unroll
-    for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
-    if (a.vpost) {
-        const C *vt = opaque(static_cast<const C *>(a.vpost));
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = v3_apply(x[e], vt, base + e * TL, a.vpost_twice);
-    }
+    axis_ops<C, L, E, FX>(x, sm, lay, lbar, t, tw, a, [=](int e) { return base + e * TL; });
     C *o = const_cast<C *>(opaque(psi));
 #pragma unroll
     for (int e = 0; e < E; ++e) st_stream(o + base + e * TL, x[e]);
@@ -127,7 +176,7 @@ __global__ void __launch_bounds__(B *(L / E)) k3_row(Pass3Args a)
 
 // strided lines (y or x): W adjacent z positions, line element i at
 // o * s_outer + c + i * s_line (blockIdx.y = o, blockIdx.x * W + lane = c)
-template <class T, int L, int E, int W>
+template <class T, int L, int E, int W, bool FX = false>
 __global__ void __launch_bounds__(W *(L / E), min_blocks3(W *(L / E))) k3_col(Pass3Args a)
 {
     pdl_wait();
@@ -146,7 +195,6 @@ __global__ void __launch_bounds__(W *(L / E), min_blocks3(W *(L / E))) k3_col(Pa
     const CtaBarrier bar{};
     C *psi = static_cast<C *>(a.psi);
     const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
-    const C *kt = static_cast<const C *>(a.k);
 
     C x[E];
 #pragma unroll
@@ -171,25 +219,7 @@ __global__ void __launch_bounds__(W *(L / E), min_blocks3(W *(L / E))) k3_col(Pa
         }
         return;
     }
-    if (a.vpre) {
-        const C *vt = opaque(static_cast<const C *>(a.vpre));
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = v3_apply(x[e], vt, base + e * stride, a.vpre_twice);
-    }
-#pragma unroll 1
-    for (int q = 0; q < 2; ++q) {
-        line_fft<C, L, E, false>(x, sm, lay, bar, t, tw);
-        if (q == 1) continue;
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = cconj(k3_apply(x[e], kt, t + e * TM, a.inv_l));
-    }
-#pragma unroll
-    for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
-    if (a.vpost) {
-        const C *vt = opaque(static_cast<const C *>(a.vpost));
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[e] = v3_apply(x[e], vt, base + e * stride, a.vpost_twice);
-    }
+    axis_ops<C, L, E, FX>(x, sm, lay, bar, t, tw, a, [=](int e) { return base + e * stride; });
     C *o = const_cast<C *>(opaque(psi));
 #pragma unroll
     for (int e = 0; e < E; ++e) st_stream(o + base + e * stride, x[e]);

@@ -12,25 +12,31 @@ constexpr int b3(int prec, int l) { return (prec == 1 ? 4096 : 2048) / l > 1 ? (
 // strided lines: W adjacent ones per CTA, W * L / E <= 512 threads, W <= 16
 constexpr int w3(int prec, int l) { return (prec == 1 ? 8192 : 4096) / l > 16 ? 16 : (prec == 1 ? 8192 : 4096) / l; }
 
-template <class T, int L>
+template <class T, int L, bool FX = false>
 static cudaError_t run3_row(size_t lines, const Pass3Args &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run3_row<T, L, true>(lines, a, st);
+    }
     constexpr int P = sizeof(T) == 4 ? 1 : 0, E = e3(P), B = b3(P, L);
     constexpr int PADS = P ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * B * padded<L, PADS>(L);
-    auto k = k3_row<T, L, E, B>;
+    auto k = k3_row<T, L, E, B, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     launch_pdl(k, dim3((unsigned)(lines / B)), dim3(B * (L / E)), smem, st, a);
     return cudaGetLastError();
 }
 
-template <class T, int L>
+template <class T, int L, bool FX = false>
 static cudaError_t run3_col(int inner, int outer, const Pass3Args &a, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run3_col<T, L, true>(inner, outer, a, st);
+    }
     constexpr int P = sizeof(T) == 4 ? 1 : 0, E = e3(P), W = w3(P, L);
     const size_t smem = sizeof(cplx_t<T>) * col_tile_elems(sizeof(cplx_t<T>), L, W, E);
-    auto k = k3_col<T, L, E, W>;
+    auto k = k3_col<T, L, E, W, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     launch_pdl(k, dim3(inner / W, outer), dim3(W * (L / E)), smem, st, a);
