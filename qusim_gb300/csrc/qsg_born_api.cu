@@ -309,8 +309,10 @@ int create_2d(qsg_born *b, const double *V)
     QSG_CUDA(cudaStreamSynchronize(b->ctx->st));
     b->g = qsg::born_split(b->prec, nx, ny);
     const int m = nx / b->g;
-    if ((rc = get_twiddles(b->ctx, b->prec, ny, qsg::born_e(b->prec), &b->tw_a))) return rc;
-    if ((rc = get_twiddles(b->ctx, b->prec, m, qsg::born_col_e(b->prec, m), &b->tw_b))) return rc;
+    const int re = qsg::born_row_e(b->prec, qsg::born_small_row(b->prec, nx, ny));
+    const int ce = qsg::born_col_e(b->prec, m, qsg::born_small_col(b->prec, nx, ny));
+    if ((rc = get_twiddles(b->ctx, b->prec, ny, re, &b->tw_a))) return rc;
+    if ((rc = get_twiddles(b->ctx, b->prec, m, ce, &b->tw_b))) return rc;
     if ((rc = get_circle(b->ctx, b->prec, nx, &b->tw_n))) return rc;
     return QSG_OK;
 }

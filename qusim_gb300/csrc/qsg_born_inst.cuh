@@ -11,9 +11,9 @@ template <class T> constexpr int born_prec() { return sizeof(T) == 4 ? 1 : 0; }
 
 // 2D row pass: B groups of G rows per CTA, B * G * NY / E >= 256 threads where
 // the rows are short (one group of G rows otherwise)
-constexpr int born_row_b(int prec, int ny, int g)
+constexpr int born_row_b(int prec, int ny, int g, bool small)
 {
-    return (prec == 1 ? 4096 : 2048) / (ny * g) > 1 ? (prec == 1 ? 4096 : 2048) / (ny * g) : 1;
+    return (256 * born_row_e(prec, small)) / (ny * g) > 1 ? (256 * born_row_e(prec, small)) / (ny * g) : 1;
 }
 // G = nx / (1024 complex64, 512 complex128 rows), at most 4, and at most
 // 512 / (ny / E) so that one group of G rows fits a CTA of 512 threads
@@ -29,9 +29,9 @@ constexpr int born_split_c(int prec, int nx, int ny)
 }
 // 2D column pass: W adjacent columns of M rows, W * M / E <= 512 threads (1024 for complex128
 // blocks of 4096 rows)
-constexpr int born_col_w(int prec, int m)
+constexpr int born_col_w(int prec, int m, bool small)
 {
-    return prec == 1 ? (m <= 512 ? 16 : (m <= 1024 ? 8 : 4))
+    return prec == 1 ? (m <= (small ? 256 : 512) ? 16 : (m <= 1024 ? 8 : 4))
                      : (m <= 256 ? 16 : (m == 512 ? 8 : (m == 1024 ? 4 : 2)));
 }
 // four-step column pass: W * N2 / E = 512 threads
@@ -42,10 +42,10 @@ constexpr int born_fs_b(int prec, int n1)
     return (prec == 1 ? 4096 : 2048) / n1 > 1 ? (prec == 1 ? 4096 : 2048) / n1 : 1;
 }
 
-template <class T, int NY, int G>
+template <class T, int NY, int G, bool SMALL>
 static cudaError_t run_born_row(int nx, const BornRowArgs &a, cudaStream_t st)
 {
-    constexpr int P = born_prec<T>(), E = born_e(P), B = born_row_b(P, NY, G);
+    constexpr int P = born_prec<T>(), E = born_row_e(P, SMALL), B = born_row_b(P, NY, G, SMALL);
     constexpr int PADS = P ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * B * G * padded<NY, PADS>(NY);
     auto k = k_born_row<T, NY, E, G, B>;
@@ -55,10 +55,13 @@ static cudaError_t run_born_row(int nx, const BornRowArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <class T, int M>
-static cudaError_t run_born_col(int ny, int g, const BornColArgs &a, cudaStream_t st)
+template <class T, int M, bool SMALL = false>
+static cudaError_t run_born_col(int ny, int g, bool small, const BornColArgs &a, cudaStream_t st)
 {
-    constexpr int P = born_prec<T>(), E = born_col_e(P, M), W = born_col_w(P, M);
+    if constexpr (sizeof(T) == 4 && !SMALL && M <= 1024) {
+        if (small) return run_born_col<T, M, true>(ny, g, small, a, st);
+    }
+    constexpr int P = born_prec<T>(), E = born_col_e(P, M, SMALL), W = born_col_w(P, M, SMALL);
     const size_t smem = sizeof(cplx_t<T>) * col_tile_elems(sizeof(cplx_t<T>), M, W, E);
     auto k = k_born_col<T, M, E, W>;
     cudaError_t e = prepare_smem(k, smem);
@@ -107,14 +110,17 @@ static cudaError_t run_born_fs_row(int n2, const BornFsRowArgs &a, cudaStream_t 
 
 #define QSG_BORN_2D_SIZES(X) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
 
-template <class T, int NY>
+template <class T, int NY, bool SMALL = false>
 static cudaError_t run_born_row_g(int nx, const BornRowArgs &a, cudaStream_t st)
 {
-    constexpr int P = born_prec<T>(), TL = NY / born_e(P);
+    constexpr int P = born_prec<T>(), TL = NY / born_row_e(P, SMALL);
+    if constexpr (sizeof(T) == 4 && !SMALL) {
+        if (born_small_row(P, nx, NY)) return run_born_row_g<T, NY, true>(nx, a, st);
+    }
     switch (born_split(P, nx, NY)) {
-    case 1: return run_born_row<T, NY, 1>(nx, a, st);
-    case 2: if constexpr (2 * TL <= 512) return run_born_row<T, NY, 2>(nx, a, st); break;
-    case 4: if constexpr (4 * TL <= 512) return run_born_row<T, NY, 4>(nx, a, st); break;
+    case 1: return run_born_row<T, NY, 1, SMALL>(nx, a, st);
+    case 2: if constexpr (2 * TL <= 512) return run_born_row<T, NY, 2, SMALL>(nx, a, st); break;
+    case 4: if constexpr (4 * TL <= 512) return run_born_row<T, NY, 4, SMALL>(nx, a, st); break;
     default: break;
     }
     return cudaErrorNotSupported;
@@ -132,7 +138,8 @@ template <class T> cudaError_t born_row(int nx, int ny, const BornRowArgs &a, cu
 template <class T> cudaError_t born_col(int nx, int ny, const BornColArgs &a, cudaStream_t st)
 {
     const int g = born_split(born_prec<T>(), nx, ny);
-#define X(N) case N: return run_born_col<T, N>(ny, g, a, st);
+    const bool small = born_small_col(born_prec<T>(), nx, ny);
+#define X(N) case N: return run_born_col<T, N>(ny, g, small, a, st);
     switch (nx / g) { QSG_BORN_2D_SIZES(X) default: break; }
 #undef X
     return cudaErrorNotSupported;

@@ -110,8 +110,15 @@ bool born1d_resident(int prec, uint64_t n);
 bool born1d_supported(int prec, uint64_t n);
 void born_fs_split(uint64_t n, int *n1, int *n2);
 
-// column-transform radix of the 2D k-space pass
-constexpr int born_col_e(int prec, int m) { return prec == 1 ? (m >= 512 ? 32 : 16) : 8; }
+// complex64 grids that leave lanes idle: half the elements per thread, so that a
+// thread runs fewer instructions in a row (per update 256^2 20.9 -> 14.0 us, 512^2
+// 25.8 -> 16.2, 1024^2 30.5 -> 27.9).  Columns up to 2^20 sites (2048^2: 95.9 us
+// wide, 101.9 so), rows up to half of that (1024^2: 27.9 wide, 30.0 so).
+constexpr bool born_small_col(int prec, int nx, int ny) { return prec == 1 && (long)nx * ny <= 1048576; }
+constexpr bool born_small_row(int prec, int nx, int ny) { return prec == 1 && (long)nx * ny <= 524288; }
+// elements per thread of the 2D row and column transforms
+constexpr int born_row_e(int prec, bool small) { return small ? 8 : born_e(prec); }
+constexpr int born_col_e(int prec, int m, bool small) { return prec == 1 ? (m >= 512 && !small ? 32 : 16) : 8; }
 // the x split of an nx x ny grid: column blocks of <= 1024 rows (complex64) /
 // 512 (complex128), as far as a CTA of G rows of ny stays within 512 threads
 int born_split(int prec, int nx, int ny);
