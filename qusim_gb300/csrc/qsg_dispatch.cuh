@@ -68,7 +68,8 @@ static inline unsigned persistent_grid(K kernel, int threads, size_t smem, int u
 // Row pass: B groups of G rows per CTA so a CTA holds >= 256 threads of line
 // work; the NT threads of a CTA (256 or 512) go over its NL = B*G lines in
 // RS = NL*(NY/E)/NT rounds (NT >= NY/E: a line is never split across rounds).
-// Plans of fewer threads (complex128, small grids) hold fewer groups instead.
+// Plans of fewer threads (complex128; complex64 rows of 1024 and 2048 points
+// without an x split) hold fewer groups instead.
 constexpr int row_b_for(int ny, int e, int g, int nt)
 {
     return ((nt < 256 ? nt : 256) / (g * (ny / e))) > 1 ? (nt < 256 ? nt : 256) / (g * (ny / e)) : 1;
@@ -88,6 +89,7 @@ constexpr size_t row_smem_for(int csz, int ny, int e, int g, int nt)
     X(T, 1024, E, 1, 256) X(T, 1024, E, 2, 256) X(T, 1024, E, 4, 256)
 #define QSG_ROW_VARIANTS_F32A(X) \
     QSG_ROW_SMALL(X, float, 16) \
+    X(float, 1024, 16, 1, 128) X(float, 2048, 16, 1, 128) \
     X(float, 2048, 16, 1, 256) X(float, 2048, 16, 2, 256) X(float, 2048, 16, 4, 256) X(float, 2048, 16, 4, 512) \
     X(float, 4096, 16, 1, 256) X(float, 4096, 16, 2, 256) X(float, 4096, 16, 2, 512) \
     X(float, 4096, 16, 4, 256) X(float, 4096, 16, 4, 512) X(float, 4096, 16, 4, 1024) \
