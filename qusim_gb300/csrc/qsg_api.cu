@@ -82,6 +82,7 @@ struct qsg_inst {
     void *vtab[2] = {nullptr, nullptr};
     void *ktab[2] = {nullptr, nullptr};  // 1D kinetic tables, or 2D fp64 full tables
     void *kx[2] = {nullptr, nullptr}, *ky[2] = {nullptr, nullptr};  // 2D complex64 separable
+    const void *tw_fx = nullptr;  // 1D Bluestein lines in fixed point
     const void *tw = nullptr, *tw_row = nullptr, *tw_col = nullptr, *tw_nx = nullptr, *tw_kin = nullptr;
     Plan2D plan{};
     Geom2D geom{};
@@ -392,7 +393,7 @@ int step1d(qsg_inst *in, uint64_t nsteps, int renorm)
     if (in->blue) {
         qsg::BlueArgs a{};
         a.psi = in->psi;
-        a.tw = in->tw;
+        a.tw = in->fx ? in->tw_fx : in->tw;
         a.w = in->fx ? in->bwf : in->bw;
         a.hs = in->fx ? in->bhsf : in->bhs;
         a.fx = in->fx ? 1 : 0;
@@ -1970,6 +1971,7 @@ static int create_1d_locked(qsg_ctx *ctx, uint64_t n, double dx, double mass, do
     int rc = QSG_OK;
     if (in->blue) {
         rc = get_twiddles(ctx, precision, blue_m, qsg::blue_elems(precision), &in->tw);
+        if (!rc && in->fx) rc = get_twiddles(ctx, precision, blue_m, qsg::blue_fx_e(blue_m), &in->tw_fx);
     } else if (!in->fourstep) {
         // the wall transforms run on the 2n odd extension
         rc = get_twiddles(ctx, precision, (int)(wall ? 2 * n : n), qsg::elems_per_thread(precision), &in->tw);

@@ -21,7 +21,7 @@ cudaError_t run_blue(const BlueArgs &a, cudaStream_t st)
     if constexpr (sizeof(T) == 8 && !FX) {
         if (a.fx) return run_blue<T, M, true>(a, st);
     }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
+    constexpr int E = FX ? blue_fx_e(M) : (sizeof(T) == 4 ? 16 : 8);
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M);
     auto k = k_evolve1d_blue<T, M, E, FX>;
