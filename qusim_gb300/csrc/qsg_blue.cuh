@@ -53,9 +53,10 @@ struct BlueArgs {
 };
 
 // 1D resident evolution of one instance of any length n (2n - 1 <= M).
-// FX (complex128, real time steps): the line stays in fixed point for all steps,
-// and the closing chirp w* of a kinetic substep cancels against the opening w of
-// the next around the V product, which then only has to zero the slots from n on.
+// FX (complex128, real time steps): the line stays in fixed point for a step, and
+// inside it the closing chirp w* of a kinetic substep cancels against the opening
+// w of the next around the V product, which then only has to zero the slots from
+// n on.
 template <class T, int M, int E, bool FX = false>
 __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
 {
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
         FixLine<M, E> f;
         f.load(x, sm, lay, bar, t);
         if (fix_flagged(tab(v0) - t + n) || (a.order == 4 && fix_flagged(tab(v1) - t + n))) f.finite = false;
-        f.mul(upto_n(tab(v0)), false);
-        f.mul([&](int e) { return __ldg(tab(w) + e * TL); }, false);
+        f.mul(upto_n(tab(v0)));
+        f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
 #pragma unroll 1
         for (uint64_t s = 0; s < a.nsteps; ++s) {
 #pragma unroll 1
@@ -142,23 +143,28 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
                 const bool last = u == nsub - 1;
                 if ((ph & 1) == 0) {
                     f.ex += a.hs_exp;
-                    f.mul([&](int e) { return __ldg(tab(hs) + e * TL); }, false);
+                    f.mul([&](int e) { return __ldg(tab(hs) + e * TL); });
                     f.conj();
                 } else if (ph == 1) {
                     const fixw *k = tab(a.order == 4 && u == 1 ? k1 : k0);
                     f.ex += a.k_exp;
                     f.conj();
-                    f.mul([&](int e) { return __ldg(k + e * TL); }, false);
+                    f.mul([&](int e) { return __ldg(k + e * TL); });
                     f.conj();
                 } else {
-                    f.mul(upto_n(tab(a.order == 4 && !last ? v1 : v0)), last && s + 1 < a.nsteps);
+                    if (last) {  // the closing chirp (elsewhere it cancels against the opening one)
+                        f.conj();
+                        f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
+                        f.conj();
+                    }
+                    f.mul(upto_n(tab(a.order == 4 && !last ? v1 : v0)));
+                    if (last && s + 1 < a.nsteps) {
+                        f.round(x, sm, lay, bar, t);
+                        f.mul(upto_n(tab(v0)));
+                        f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
+                    }
                 }
             }
-        }
-        if (a.nsteps) {
-            f.conj();
-            f.mul([&](int e) { return __ldg(tab(w) + e * TL); }, false);
-            f.conj();
         }
         f.store(x);
     } else {
@@ -347,29 +353,35 @@ __global__ void __launch_bounds__(RPC *(M / E), FX && RPC * (M / E) <= 256 ? 768
         if (bad) f.finite = false;
         if (a.in_k) {
             f.conj();
-            f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+            f.mul([&](int e) { return __ldg(wf + e * TL); });
         }
         const int npass = 2 * ((a.in_k ? 1 : 0) + (a.out_k ? 1 : 0)), vpos = a.in_k ? 2 : 0;
 #pragma unroll 1
         for (int p = 0; p <= npass; ++p) {
             if (p > 0) f.scale(sm, lay, bar, t);
             if (p == vpos) {
-                if (a.in_k && !a.out_k) {  // the inverse DFT's closing w* (out_k: cancels against the opening w)
+                // inside a step the inverse DFT's closing w* cancels against the opening w; where a
+                // step ends (V twice) the line is rounded as a call's end would
+                const bool cancel = a.in_k && a.out_k && !a.vtwice;
+                auto v_row = [&](int e) { return t + e * TL < ny ? ld_stream(vr + e * TL) : fixw{0, 0, 0, 0}; };
+                if (a.in_k && !cancel) {
                     f.conj();
-                    f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+                    f.mul([&](int e) { return __ldg(wf + e * TL); });
                     f.conj();
                 }
-                if (vt)
-                    f.mul([&](int e) { return t + e * TL < ny ? ld_stream(vr + e * TL) : fixw{0, 0, 0, 0}; },
-                          a.vtwice != 0);
-                if (a.out_k && !a.in_k) f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+                if (vt) f.mul(v_row);
+                if (vt && a.vtwice) {
+                    f.round(x, sm, lay, bar, t);
+                    f.mul(v_row);
+                }
+                if (a.out_k && !cancel) f.mul([&](int e) { return __ldg(wf + e * TL); });
             } else if (p & 1) {
                 f.ex += a.hs_exp;
-                f.mul([&](int e) { return __ldg(hf + e * TL); }, false);
+                f.mul([&](int e) { return __ldg(hf + e * TL); });
                 f.conj();
             } else if (p == npass) {
                 f.conj();
-                f.mul([&](int e) { return __ldg(wf + e * TL); }, false);
+                f.mul([&](int e) { return __ldg(wf + e * TL); });
             }
             if (p < npass) f.fft(sm, lay, bar, t, opaque(tw));
         }
@@ -441,24 +453,24 @@ __global__ void __launch_bounds__(W *(M / E), FX && W * (M / E) <= 512 ? 1024 / 
         const fixw kyf = __ldg(static_cast<const fixw *>(a.ky) + (active ? col : 0));
         FixLine<M, E> f;
         f.load(x, sm, lay, bar, t);
-        f.mul([&](int e) { return __ldg(wf + e * TM); }, false);
+        f.mul([&](int e) { return __ldg(wf + e * TM); });
 #pragma unroll 1
         for (int p = 0; p < 4; ++p) {
             f.fft(sm, lay, bar, t, opaque(tw));
             f.scale(sm, lay, bar, t);
             if ((p & 1) == 0) {
                 f.ex += a.hs_exp;
-                f.mul([&](int e) { return __ldg(hf + e * TM); }, false);
+                f.mul([&](int e) { return __ldg(hf + e * TM); });
                 f.conj();
             } else if (p == 1) {
                 f.ex += a.k_exp;
                 f.conj();
-                f.mul([&](int e) { return t + e * TM < nx ? __ldg(kx + e * TM) : fixw{0, 0, 0, 0}; }, false);
-                f.mul([&](int) { return kyf; }, false);
+                f.mul([&](int e) { return t + e * TM < nx ? __ldg(kx + e * TM) : fixw{0, 0, 0, 0}; });
+                f.mul([&](int) { return kyf; });
                 f.conj();
             } else {
                 f.conj();
-                f.mul([&](int e) { return __ldg(wf + e * TM); }, false);
+                f.mul([&](int e) { return __ldg(wf + e * TM); });
                 f.conj();
             }
         }

@@ -76,7 +76,8 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
         auto mul_v = [&](const void *v, bool twice) {
             const fixw *vt = opaque(static_cast<const fixw *>(v));
             if (fix_flagged(vt + a.n)) f.finite = false;
-            f.mul([&](int e) { return ld_stream(vt + idx(e)); }, twice);
+            f.mul([&](int e) { return ld_stream(vt + idx(e)); });
+            if (twice) f.mul([&](int e) { return ld_stream(vt + idx(e)); });
         };
         if (a.v[0]) mul_v(a.v[0], false);
 #pragma unroll 1
@@ -86,7 +87,7 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
             if ((q & 1) == 0) {
                 const fixw *kt = static_cast<const fixw *>(q ? a.k2 : a.k);
                 f.ex -= Plan<L, E>::LOGL;  // 1/L
-                f.mul([&](int e) { return __ldg(kt + t + e * TL); }, false);
+                f.mul([&](int e) { return __ldg(kt + t + e * TL); });
                 f.conj();
             } else {
                 f.conj();

@@ -311,22 +311,25 @@ template <int L, int E> struct FixLine {
         fix_norm(v, Red::get(m, w + r), ex);
         if constexpr (!Red::WARP) r = after(r);
     }
-    // v *= f(e), `twice`: two products (the reference's two multiplies by one table value);
-    // H < E: only the first H slots (the others are not used afterwards)
-    template <int H = E, class F> __device__ __forceinline__ void mul(F f, bool twice)
+    // v *= f(e); H < E: only the first H slots (the others are not used afterwards)
+    template <int H = E, class F> __device__ __forceinline__ void mul(F f)
     {
-        if (twice) {
 #pragma unroll
-            for (int e = 0; e < H; ++e) {
-                const fixw m = f(e);
-                v[e] = fix_twmul(fix_twmul(v[e], m), m);
-            }
-            ex += 4;
-        } else {
+        for (int e = 0; e < H; ++e) v[e] = fix_twmul(v[e], f(e));
+        ex += 2;
+    }
+    // The end of a step: the line rounded to doubles and taken up again, as a call that ended
+    // here would store it and the next one load it (H < E: slots from H on zero).  A step split
+    // across calls, chunks of the server or reads of the state then equals one call bit for bit.
+    template <int H = E, class Lay, class Bar>
+    __device__ __forceinline__ void round(double2 (&x)[E], double2 *smd, const Lay &lay, const Bar &bar, int t)
+    {
+        const bool ok = finite;
+        store(x);
 #pragma unroll
-            for (int e = 0; e < H; ++e) v[e] = fix_twmul(v[e], f(e));
-            ex += 2;
-        }
+        for (int e = H; e < E; ++e) x[e] = double2{0, 0};
+        load(x, smd, lay, bar, t);
+        finite = finite && ok;
     }
     // the product's change of scale without a product
     __device__ __forceinline__ void quarter()

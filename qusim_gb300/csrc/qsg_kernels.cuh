@@ -329,7 +329,11 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
                     }
                     if (vt) {
                         const fixw *vr = opaque(reinterpret_cast<const fixw *>(vt)) + (size_t)row * NY + t;
-                        f.mul([&](int e) { return ld_stream(vr + e * TL); }, a.vtwice != 0);
+                        f.mul([&](int e) { return ld_stream(vr + e * TL); });
+                        if (a.vtwice) {
+                            f.round(x, sm, lay, lbar, t);
+                            f.mul([&](int e) { return ld_stream(vr + e * TL); });
+                        }
                     } else {
                         f.quarter();
                     }
@@ -545,7 +549,7 @@ __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : si
             if (p == 0) {
                 f.scale(sm, lay, bar, t);
                 const fixw *k2 = opaque(static_cast<const fixw *>(a.k2d)) + col;
-                f.mul([&](int e) { return ld_stream(k2 + (size_t)(a.g * (t + e * TM) + q) * ny); }, false);
+                f.mul([&](int e) { return ld_stream(k2 + (size_t)(a.g * (t + e * TM) + q) * ny); });
             }
             f.conj();
         }
@@ -796,7 +800,7 @@ __global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T)
         if (vt && fix_flagged(vt + (size_t)N2 * n1)) f.finite = false;
         if (in_k) {
             f.conj();
-            f.mul([&](int e) { return __ldg(wn + e * stride); }, false);
+            f.mul([&](int e) { return __ldg(wn + e * stride); });
         }
         const int npass = (in_k ? 1 : 0) + (out_k ? 1 : 0);
         const int vpos = in_k ? 1 : 0;
@@ -809,7 +813,11 @@ __global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T)
                 }
                 if (vt) {
                     const fixw *vr = opaque(vt) + base;
-                    f.mul([&](int e) { return ld_stream(vr + e * stride); }, a.vtwice != 0);
+                    f.mul([&](int e) { return ld_stream(vr + e * stride); });
+                    if (a.vtwice) {
+                        f.round(x, sm, lay, bar, t);
+                        f.mul([&](int e) { return ld_stream(vr + e * stride); });
+                    }
                 } else {
                     f.quarter();
                 }
@@ -820,7 +828,7 @@ __global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T)
         if (out_k) {
             f.scale(sm, lay, bar, t);
             const fixw *wo = opaque(wn);
-            f.mul([&](int e) { return __ldg(wo + e * stride); }, false);
+            f.mul([&](int e) { return __ldg(wo + e * stride); });
         }
         f.store(x);
         if (!out_k) {
@@ -930,7 +938,7 @@ __global__ void __launch_bounds__(B *(N1 / E), FX && B * (N1 / E) <= 256 ? 768 /
             if (p == 0) {
                 f.scale(sm, lay, lbar, t);
                 const fixw *kt = opaque(static_cast<const fixw *>((a.ksel ? in.ktab[1] : in.ktab[0]))) + base;
-                f.mul([&](int e) { return ld_stream(kt + e * TL); }, false);
+                f.mul([&](int e) { return ld_stream(kt + e * TL); });
             }
             if (p == 0) f.conj();
         }
@@ -1060,7 +1068,7 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
         f.load(x, sm, lay, bar, t);
         auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
         if (fix_flagged(tab(v0) - t + L) || (a.order == 4 && fix_flagged(tab(v1) - t + L))) f.finite = false;
-        f.mul([&](int e) { return __ldg(tab(v0) + e * TL); }, false);
+        f.mul([&](int e) { return __ldg(tab(v0) + e * TL); });
         for (uint64_t s = 0; s < nsteps; ++s) {
 #pragma unroll 1
             for (int h = 0; h < 2 * nsub; ++h) {
@@ -1073,8 +1081,12 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
                     f.ex -= Plan<L, E>::LOGL;  // 1/N
                 else
                     f.conj();
-                f.mul([&](int e) { return __ldg(m + e * TL); }, !kin && last && s + 1 < nsteps);
+                f.mul([&](int e) { return __ldg(m + e * TL); });
                 if (kin) f.conj();
+                if (!kin && last && s + 1 < nsteps) {
+                    f.round(x, sm, lay, bar, t);
+                    f.mul([&](int e) { return __ldg(m + e * TL); });
+                }
             }
         }
         f.store(x);
@@ -1272,7 +1284,7 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
         f.load(x, sm, lay, bar, t);
         auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
         if (fix_flagged(tab(v0) - t + L2 / 2) || (a.order == 4 && fix_flagged(tab(v1) - t + L2 / 2))) f.finite = false;
-        f.template mul<H>([&](int e) { return __ldg(tab(v0) + e * TL); }, false);
+        f.template mul<H>([&](int e) { return __ldg(tab(v0) + e * TL); });
         for (uint64_t s = 0; s < nsteps; ++s) {
 #pragma unroll 1
             for (int h = 0; h < 2 * nsub; ++h) {
@@ -1286,7 +1298,11 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
                 const bool last = u == nsub - 1, kin = (h & 1) == 0;
                 const fixw *m = tab(kin ? (a.order == 4 && u == 1 ? k1 : k0) : (a.order == 4 && !last ? v1 : v0));
                 if (kin) f.ex -= Plan<L2, E>::LOGL;  // 1/(2N); the table carries the sign
-                f.template mul<H>([&](int e) { return __ldg(m + e * TL); }, !kin && last && s + 1 < nsteps);
+                f.template mul<H>([&](int e) { return __ldg(m + e * TL); });
+                if (!kin && last && s + 1 < nsteps) {
+                    f.template round<H>(x, sm, lay, bar, t);
+                    f.template mul<H>([&](int e) { return __ldg(m + e * TL); });
+                }
             }
         }
         f.store(x);

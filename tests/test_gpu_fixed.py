@@ -147,3 +147,34 @@ def test_every_2d_plan_vs_oracle(qsg, ctx, oracle, shape):
             inst.step(1)
             got = inst.get_psi()
             assert rel_l2(got, ref) <= TOL, (dt, plan.g, plan.row_e, plan.row_nt, plan.col_e, plan.col_w)
+
+
+# complex128 steps with a real dt: split calls, and reads in between, leave the state as one call does
+# (Bluestein lines on the four-step passes apply other table values at a call's ends and agree to rounding)
+@pytest.mark.parametrize("n,wall", [(64, 0), (4096, 0), (1000, 0), (300, 0), (16384, 0), (512, 1), (700, 1), (8192, 1)])
+@pytest.mark.parametrize("order", [2, 4])
+def test_split_calls_equal_one_call(qsg, ctx, n, wall, order):
+    psi, V = line(n, "noise")
+    bc = qsg.BoundaryCondition.InfiniteWall if wall else qsg.BoundaryCondition.Period
+    a = qsg.Instance.create_1d(ctx, psi, V, 0.1, 0.01, order=order, boundary=bc)
+    b = qsg.Instance.create_1d(ctx, psi, V, 0.1, 0.01, order=order, boundary=bc)
+    a.step(7)
+    for k in (3, 1, 3):
+        b.step(k)
+        b.get_psi()
+    assert np.array_equal(a.get_psi(), b.get_psi())
+
+
+@pytest.mark.parametrize("shape", [(128, 128), (1024, 256), (4096, 128), (45, 100), (100, 128)])
+@pytest.mark.parametrize("order", [2, 4])
+def test_split_calls_equal_one_call_2d(qsg, ctx, shape, order):
+    rng = np.random.default_rng(3)
+    psi = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    V = rng.uniform(-1, 1, shape)
+    a = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, 0.01, order=order)
+    b = qsg.Instance.create_2d(ctx, psi, V, 0.1, 0.1, 0.01, order=order)
+    a.step(4)
+    for k in (1, 2, 1):
+        b.step(k)
+        b.get_psi()
+    assert np.array_equal(a.get_psi(), b.get_psi())
