@@ -776,13 +776,13 @@ def run_3d(args, w):
     ctx.profile(False)
     value = whole_job_rate(sites * args.steps, world, ms / 1e3)
     sc = 8 if args.precision == "mixed" else 16
-    # O4: 9 line passes of psi in and out, 3 of them also read a V table
-    step_b = (9 * 2 + 3) * sc if w["order"] == 4 else (3 * 2 + 1) * sc
+    # two passes of psi in and out per kinetic substep, one of which also reads a V table
+    step_b = 3 * (2 * 2 + 1) * sc if w["order"] == 4 else (2 * 2 + 1) * sc
     peak, peak_kind = measured_peaks()
     dom = max(prof.items(), key=lambda kv: kv[1][1])
     nl, tot = dom[1]
-    # x passes: 3 per step, two of them with a V table
-    per_launch = (2 * sc + (2 * sc / 3 if dom[0] == "pass3_x" else 0)) * sites
+    # x and z passes apply V between two kinetic factors of their axis; y passes read no table
+    per_launch = (2 * sc + (0 if dom[0] == "pass3_y" else sc)) * sites
     ach = per_launch / (tot / nl / 1e3) / 1e9
     roof = {"bound": "hbm", "kernel": dom[0], "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "peak_source": peak_kind, "avg_launch_ms": tot / nl, "algorithmic_bytes_per_launch": per_launch,
