@@ -776,13 +776,14 @@ def run_3d(args, w):
     ctx.profile(False)
     value = whole_job_rate(sites * args.steps, world, ms / 1e3)
     sc = 8 if args.precision == "mixed" else 16
-    # two passes of psi in and out per kinetic substep, one of which also reads a V table
-    step_b = 3 * (2 * 2 + 1) * sc if w["order"] == 4 else (2 * 2 + 1) * sc
+    # passes of psi in and out and the V tables they read: O4 six and three (each axis twice, once with a
+    # table), O2 three and one (z; complex128 with a real time step also x)
+    v_reads = {"pass3_z": 1, "pass3_y": 0, "pass3_x": 0 if args.precision == "mixed" else 1}
+    step_b = (6 * 2 + 3) * sc if w["order"] == 4 else (3 * 2 + sum(v_reads.values())) * sc
     peak, peak_kind = measured_peaks()
     dom = max(prof.items(), key=lambda kv: kv[1][1])
     nl, tot = dom[1]
-    # x and z passes apply V between two kinetic factors of their axis; y passes read no table
-    per_launch = (2 * sc + (0 if dom[0] == "pass3_y" else sc)) * sites
+    per_launch = (2 + (0.5 if w["order"] == 4 else v_reads.get(dom[0], 0))) * sc * sites
     ach = per_launch / (tot / nl / 1e3) / 1e9
     roof = {"bound": "hbm", "kernel": dom[0], "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "peak_source": peak_kind, "avg_launch_ms": tot / nl, "algorithmic_bytes_per_launch": per_launch,

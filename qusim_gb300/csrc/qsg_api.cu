@@ -701,29 +701,25 @@ int step2d(qsg_inst *in, uint64_t nsteps, int renorm)
     return QSG_OK;
 }
 
-// One 3D pass over the lines of an axis (0 x, 1 y, 2 z) of the planes
-// [x0, x0 + planes) of the first axis (all of them for axis 0):
-// [v0] F^-1 K F [v1] [F^-1 K' F] [v2]; kt, kt2: kinetic tables (kt2 < 0: none)
+// One 3D pass over the lines of an axis (0 x, 1 y, 2 z):
+// [v0] F^-1 K F [v1] [F^-1 K' F]; kt, kt2: kinetic tables (kt2 < 0: none)
 struct Pass3 {
     int ax, kt, kt2 = -1;
-    const void *v0 = nullptr, *v1 = nullptr, *v2 = nullptr;
-    bool twice = false;  // v1 applied twice
+    const void *v0 = nullptr, *v1 = nullptr;
+    bool twice = false;  // v1 (v0 where there is no second factor) applied twice
 };
-template <class T> int pass3(qsg_inst *in, const Pass3 &p, int x0, int planes, double *kin = nullptr)
+template <class T> int pass3(qsg_inst *in, const Pass3 &p, double *kin = nullptr)
 {
     qsg::Pass3Args a{};
     const int nx = in->nx, ny = in->ny, nz = in->nz;
-    const size_t off = (size_t)x0 * ny * nz * csize(in->prec);
-    auto at = [&](const void *q) { return q ? static_cast<const char *>(q) + off : nullptr; };
-    a.psi = static_cast<char *>(in->psi) + off;
-    a.v[0] = at(p.v0);
-    a.v[1] = at(p.v1);
-    a.v[2] = at(p.v2);
-    a.vmid_twice = p.twice ? 1 : 0;
+    a.psi = in->psi;
+    a.v[0] = p.v0;
+    a.v[1] = p.v1;
+    a.v_twice = p.twice ? 1 : 0;
     a.k = in->k3[p.ax][p.kt];
     a.k2 = p.kt2 >= 0 ? in->k3[p.ax][p.kt2] : nullptr;
     a.fx = in->fx ? 1 : 0;
-    a.n = in->n - (size_t)x0 * ny * nz;
+    a.n = in->n;
     a.tw = in->tw3[p.ax];
     a.partials = kin;
     a.kinetic = kin ? 1 : 0;
@@ -731,12 +727,12 @@ template <class T> int pass3(qsg_inst *in, const Pass3 &p, int x0, int planes, d
     a.inv_l = (float)(1.0 / L[p.ax]);
     if (p.ax == 2) {
         ProfScope ps(in->ctx, "pass3_z", in->st);
-        QSG_CUDA(qsg::launch3_row<T>(nz, (size_t)planes * ny, a, in->st));
+        QSG_CUDA(qsg::launch3_row<T>(nz, (size_t)nx * ny, a, in->st));
     } else if (p.ax == 1) {
         a.s_line = nz;
         a.s_outer = (long long)ny * nz;
         ProfScope ps(in->ctx, "pass3_y", in->st);
-        QSG_CUDA(qsg::launch3_col<T>(ny, nz, planes, a, in->st));
+        QSG_CUDA(qsg::launch3_col<T>(ny, nz, nx, a, in->st));
     } else {
         a.s_line = (long long)ny * nz;
         a.s_outer = nz;
@@ -746,29 +742,49 @@ template <class T> int pass3(qsg_inst *in, const Pass3 &p, int x0, int planes, d
     return QSG_OK;
 }
 
-// The passes of a call (qsg_evolve3d.cuh): z[V, K] y x[K, V, K] y z[K, V, K] y ... [K, V].
+// The passes of a call (qsg_evolve3d.cuh).
 template <class T> int step3d_t(qsg_inst *in, uint64_t nsteps)
 {
     const void *V0 = in->vtab[0], *V1 = in->vtab[1];
-    const uint64_t nsub = in->order == 2 ? 1 : 3, subs = nsteps * nsub;
-    auto kt = [&](uint64_t i) { return in->order == 4 && i % 3 == 1 ? 1 : 0; };  // O4: K1 K2 K1
-    if (subs == 0) return QSG_OK;
-    int rc;
-    Pass3 first{2, kt(0)};
-    first.v0 = V0;
-    if ((rc = pass3<T>(in, first, 0, in->nx))) return rc;
-    for (uint64_t i = 0; i < subs; ++i) {
-        if ((rc = pass3<T>(in, Pass3{1, kt(i)}, 0, in->nx))) return rc;
-        Pass3 p{i % 2 == 0 ? 0 : 2, kt(i)};
-        const bool join = i % nsub == nsub - 1;  // the step's last substep
-        p.v1 = in->order == 4 && !join ? V1 : V0;
-        if (i + 1 < subs) {
-            p.kt2 = kt(i + 1);
-            p.twice = join;  // the step's closing factor and the next one's opening factor
+    int rc = QSG_OK;
+    auto pass = [&](const Pass3 &p) {
+        if (!rc) rc = pass3<T>(in, p);
+    };
+    for (uint64_t s = 0; s < nsteps && !rc; ++s) {
+        const bool last = s + 1 == nsteps;
+        Pass3 p{2, 0};
+        if (in->order == 2) {
+            // fixed point: the closing factor stays in the x pass, whose lines it is rounded with
+            // at a call's end
+            const bool merge = s > 0 && !in->fx;
+            p.v0 = V0;
+            p.twice = merge;
+            pass(p);
+            pass(Pass3{1, 0});
+            p = Pass3{0, 0};
+            p.v1 = last || in->fx ? V0 : nullptr;
+            pass(p);
+            continue;
         }
-        if ((rc = pass3<T>(in, p, 0, in->nx))) return rc;
+        if (s == 0) {
+            p.v0 = V0;
+            pass(p);
+        }
+        pass(Pass3{1, 0});
+        p = Pass3{0, 0, 1};
+        p.v1 = V1;
+        pass(p);
+        pass(Pass3{2, 1});
+        p = Pass3{1, 1, 0};
+        p.v1 = V1;
+        pass(p);
+        pass(Pass3{0, 0});
+        p = Pass3{2, 0, last ? -1 : 0};
+        p.v1 = V0;
+        p.twice = !last;
+        pass(p);
     }
-    return QSG_OK;
+    return rc;
 }
 
 int step3d(qsg_inst *in, uint64_t nsteps, int renorm)
@@ -795,8 +811,8 @@ int kinetic3d(qsg_inst *in, double *kin)
     for (int ax = 0; ax < 3; ++ax) {
         const int ctas = ax == 2 ? qsg::row3_ctas(in->prec, in->nz, (size_t)in->nx * in->ny)
                                  : qsg::col3_ctas(in->prec, L[ax], in->nz, ax == 1 ? in->nx : in->ny);
-        int rc = in->prec == 1 ? pass3<float>(in, Pass3{ax, 0}, 0, in->nx, in->kparts3)
-                               : pass3<double>(in, Pass3{ax, 0}, 0, in->nx, in->kparts3);
+        int rc = in->prec == 1 ? pass3<float>(in, Pass3{ax, 0}, in->kparts3)
+                               : pass3<double>(in, Pass3{ax, 0}, in->kparts3);
         if (rc) return rc;
         std::vector<double> h(2 * (size_t)ctas);
         QSG_CUDA(cudaMemcpyAsync(h.data(), in->kparts3, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->st));

@@ -9,15 +9,27 @@
 // of three commuting one-axis operators F_a^-1 K_a F_a: each is a pass over the
 // lines along its axis (transform, factor, inverse transform, all on chip), and
 // V multiplies fuse into the passes.  A step never leaves natural real-space
-// layout.  Because the axes commute, a kinetic substep may take them in either
-// order: substeps alternate z y x and x y z, and the last axis of one, the V
-// between and the same axis of the next are one pass of four transforms.  With
-// s substeps in a call (1 per step in O2, 3 in O4) that is 2 s + 1 passes:
+// layout.  Because the axes commute, a kinetic substep may take them in any
+// order.  An order-4 step takes z y x, x z y, y x z: each substep starts on the
+// axis that the one before it ended on, the next step too, and the last axis of
+// one, the V between and the same axis of the next are one pass of four
+// transforms:
 //
-//   z[V, Kz] y[Ky] x[Kx, V, Kx] y[Ky] z[Kz, V, Kz] y[Ky] x[Kx, V, Kx] ... [K, V]
+//   O4: z[V1 V1', K1] y[K1] x[K1, V2, K2] z[K2] y[K2, V2, K1] x[K1] (z[K1, V1])
+//       6 passes a step, and one more that closes a call
+//   O2: z[V V', K] y[K] x[K, (V)]
+//       3 passes: one substep cannot start and end on the same axis
 //
-// against 3 s of one axis each (O4 per step: 256^3 complex64 747 -> 602 us,
-// complex128 with the products in fixed point as well 16.5 -> 3.61 ms).
+// (V' = the previous step's closing factor; in O4 its pass is also the previous
+// step's last, z[K1, V1', V1, K1]; (.) only at a call's end.)  Every step is the
+// same sequence of operations on the state wherever a call begins or ends, so
+// calls that split a run leave the state of one call bit for bit.  (Orders that
+// alternate between z y x and x y z would join O2 steps too, 2 passes a step, but
+// then a step's rounding depends on how many came before it: 226 against 243 us
+// a step at 256^3 complex64, 1.28 against 1.37 ms complex128, 8.4 against 11.1 at
+// 32^3.)  O4 against nine passes of one axis each, per step of 256^3: complex64
+// 778 -> 618 us, complex128 with the products in fixed point as well 16.6 -> 3.69
+// ms.
 // z lines are contiguous (k3_row); y and x lines are strided by nz and ny*nz
 // (k3_col, W adjacent z positions per CTA so every access is a W-wide contiguous
 // segment).
@@ -28,9 +40,11 @@ namespace qsg {
 
 struct Pass3Args {
     void *psi;
-    const void *v[3];      // V factor before the axis operator, after it (before a second one),
-                           // after the second (or null each); natural layout, n entries
-    int vmid_twice;        // v[1] applied twice (the two ExpV calls at a step boundary)
+    const void *v[2];      // V factor before the axis operator and after it (or null each; with a
+                           // second axis factor the one between the two, not null); natural layout,
+                           // n entries
+    int v_twice;           // the two ExpV calls at a step boundary: v[1] applied twice where there is a
+                           // second axis factor, v[0] otherwise (not with FX)
     const void *k, *k2;    // the axis factor, and a second one (or null): complex64 factor - 1,
                            // complex128 factor / L (FX: fixed-point factors)
     int fx;
@@ -61,7 +75,7 @@ template <class C> __device__ __forceinline__ C k3_apply(C x, const C *kt, int k
     else return cmul(x, ld_c(kt + k));
 }
 
-// [V] F^-1 K F [V] [F^-1 K2 F] [V] on a line in registers, the inverse as
+// [V] F^-1 K F [V] [F^-1 K2 F] on a line in registers, the inverse as
 // conj(F(conj(.))); idx(e): the site of slot e.  One transform body in a loop.
 // FX (complex128, real time steps): the line is in fixed point throughout.
 template <class C, int L, int E, bool FX, class Lay, class Bar, class I>
@@ -77,7 +91,10 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
             const fixw *vt = opaque(static_cast<const fixw *>(v));
             if (fix_flagged(vt + a.n)) f.finite = false;
             f.mul([&](int e) { return ld_stream(vt + idx(e)); });
-            if (twice) f.mul([&](int e) { return ld_stream(vt + idx(e)); });
+            if (twice) {  // between two steps: rounded as a call's end would
+                f.round(x, sm, lay, bar, t);
+                f.mul([&](int e) { return ld_stream(vt + idx(e)); });
+            }
         };
         if (a.v[0]) mul_v(a.v[0], false);
 #pragma unroll 1
@@ -91,16 +108,12 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
                 f.conj();
             } else {
                 f.conj();
-                const void *v = q == 1 ? a.v[1] : a.v[2];
-                if (v)
-                    mul_v(v, q == 1 && a.vmid_twice);
-                else if (q + 1 < nq)
-                    f.quarter();
+                if (q == 1 && a.v[1]) mul_v(a.v[1], a.v_twice);
             }
         }
         f.store(x);
     } else {
-        if (a.v[0]) v3_apply(x, a.v[0], idx, false);
+        if (a.v[0]) v3_apply(x, a.v[0], idx, a.v_twice && !a.k2);
 #pragma unroll 1
         for (int q = 0; q < nq; ++q) {
             line_fft<C, L, E, false>(x, sm, lay, bar, t, tw);
@@ -111,8 +124,7 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
             } else {
 #pragma unroll
                 for (int e = 0; e < E; ++e) x[e] = cconj(x[e]);
-                const void *v = q == 1 ? a.v[1] : a.v[2];
-                if (v) v3_apply(x, v, idx, q == 1 && a.vmid_twice);
+                if (q == 1 && a.v[1]) v3_apply(x, a.v[1], idx, a.v_twice && a.k2);
             }
         }
     }
