@@ -98,7 +98,7 @@ template <> __device__ __forceinline__ float2 phase_entry<float2>(double x, doub
 // units of 2^-62 (in integers: FP64 roundings cost a tenth of the table build).
 __device__ __forceinline__ int2 fix_part(double c)
 {
-    const long long v = fix_from(c, 1023, 10);
+    const long long v = fix_from<10>(c, 1023);
     const int l = fix_lo(v);
     return make_int2(fix_hir(v), l == (int)0x80000000 ? l + 1 : l);
 }

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
         FixLine<M, E> f;
         f.load(x, sm, lay, bar, t);
         if (fix_flagged(tab(v0) - t + n) || (a.order == 4 && fix_flagged(tab(v1) - t + n))) f.finite = false;
-        f.mul(upto_n(tab(v0)));
+        f.mul_full(upto_n(tab(v0)));
         f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
 #pragma unroll 1
         for (uint64_t s = 0; s < a.nsteps; ++s) {
@@ -154,13 +154,13 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
                 } else {
                     if (last) {  // the closing chirp (elsewhere it cancels against the opening one)
                         f.conj();
-                        f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
+                        f.mul_full([&](int e) { return __ldg(tab(w) + e * TL); });
                         f.conj();
                     }
-                    f.mul(upto_n(tab(a.order == 4 && !last ? v1 : v0)));
+                    f.mul_v(upto_n(tab(a.order == 4 && !last ? v1 : v0)));
                     if (last && s + 1 < a.nsteps) {
                         f.round(x, sm, lay, bar, t);
-                        f.mul(upto_n(tab(v0)));
+                        f.mul_full(upto_n(tab(v0)));
                         f.mul([&](int e) { return __ldg(tab(w) + e * TL); });
                     }
                 }
@@ -366,13 +366,16 @@ __global__ void __launch_bounds__(RPC *(M / E), FX && RPC * (M / E) <= 256 ? 768
                 auto v_row = [&](int e) { return t + e * TL < ny ? ld_stream(vr + e * TL) : fixw{0, 0, 0, 0}; };
                 if (a.in_k && !cancel) {
                     f.conj();
-                    f.mul([&](int e) { return __ldg(wf + e * TL); });
+                    f.mul_full([&](int e) { return __ldg(wf + e * TL); });
                     f.conj();
                 }
-                if (vt) f.mul(v_row);
-                if (vt && a.vtwice) {
-                    f.round(x, sm, lay, bar, t);
-                    f.mul(v_row);
+                if (vt && cancel) f.mul_v(v_row);
+                if (vt && !cancel) {  // the closing w or the pass's end follows
+#pragma unroll 1
+                    for (int k = 0; k <= a.vtwice; ++k) {
+                        if (k) f.round(x, sm, lay, bar, t);
+                        f.mul_full(v_row);
+                    }
                 }
                 if (a.out_k && !cancel) f.mul([&](int e) { return __ldg(wf + e * TL); });
             } else if (p & 1) {
@@ -465,7 +468,7 @@ __global__ void __launch_bounds__(W *(M / E), FX && W * (M / E) <= 512 ? 1024 / 
             } else if (p == 1) {
                 f.ex += a.k_exp;
                 f.conj();
-                f.mul([&](int e) { return t + e * TM < nx ? __ldg(kx + e * TM) : fixw{0, 0, 0, 0}; });
+                f.mul_full([&](int e) { return t + e * TM < nx ? __ldg(kx + e * TM) : fixw{0, 0, 0, 0}; });
                 f.mul([&](int) { return kyf; });
                 f.conj();
             } else {

@@ -90,10 +90,10 @@ __device__ __forceinline__ void axis_ops(C (&x)[E], C *sm, const Lay &lay, const
         auto mul_v = [&](const void *v, bool twice) {
             const fixw *vt = opaque(static_cast<const fixw *>(v));
             if (fix_flagged(vt + a.n)) f.finite = false;
-            f.mul([&](int e) { return ld_stream(vt + idx(e)); });
+            f.mul_v([&](int e) { return ld_stream(vt + idx(e)); });
             if (twice) {  // between two steps: rounded as a call's end would
                 f.round(x, sm, lay, bar, t);
-                f.mul([&](int e) { return ld_stream(vt + idx(e)); });
+                f.mul_v([&](int e) { return ld_stream(vt + idx(e)); });
             }
         };
         if (a.v[0]) mul_v(a.v[0], false);

@@ -8,16 +8,17 @@
 // butterflies add 64-bit integers exactly, the twiddle products round to the
 // last place, and the line goes back to double at the end.
 //
-// Precision.  The largest component of a line is kept between 2^57 and 2^61
-// units of the fixed point (re-scaled after a stage by the largest magnitude the
-// stage left, a reduction that rides on the exchange's barrier), so every
-// rounding is at most 2^-57 of the line's largest value, where a double's is
-// 2^-53 of each value.  An FFT's error is relative to the line's norm in either
-// arithmetic.  Against 80-bit runs of the same steps the error fell on every
-// shape tried (1D 64 .. 131072, Bluestein and wall lines, 2D 128^2 .. 512^2,
-// packets and white noise): 0.12 to 0.8 of the FP64 transforms' error, e.g.
-// 1.4e-14 -> 3.6e-15 after 30 O4 steps at n = 4096.
-//
+// Precision.  Before a product the largest component of a line is between 2^57
+// and 2^61 units (re-scaled after a stage by the largest magnitude the stage left,
+// a reduction that rides on the exchange's barrier).  A product divides by four
+// and is off by at most one unit of its result (half a unit of rounding, half of
+// the low words' product left out), so by at most 2^-55 of the line's largest
+// component, and by 2^-56.7 rms where that sits at 2^57 (2^-60.7 at 2^61).  Two
+// products in a row keep that bound: the first one does not divide (mul_full).
+// Taking a line up from doubles rounds to nearest, at 2^-59 of its largest
+// component.  A double's rounding is 2^-53 of each value; a small component of a
+// line has fewer significant bits here, but an FFT's error is relative to the
+// line's norm in either arithmetic.
 // A unit-modulus factor w is stored as {re hi, re lo, im hi, im lo}: hi =
 // round(w 2^30), lo = the rest at 2^-62, so w is held to 2^-63.
 #pragma once
@@ -39,14 +40,27 @@ __device__ __forceinline__ int fix_hir(long long v) { return fix_hi(v) + (int)((
 // c + a b in 64 bits (IMAD.WIDE)
 __device__ __forceinline__ long long fix_mad(int a, int b, long long c) { return (long long)a * b + c; }
 
+// v / 2^r, rounded to nearest, halves to even (r = 1, 2: a fixed direction would
+// be a drift of an eighth to a quarter of a unit per rounding)
+__device__ __forceinline__ long long fix_shr(long long v, int r)
+{
+    return (v + ((1 << (r - 1)) - 1 + ((fix_lo(v) >> r) & 1))) >> r;
+}
+
 // a w / 4 for |a.x|, |a.y| < 2^61.  With a = h 2^32 + l and w = wh 2^-30 + wl 2^-62,
 // a w / 4 = h wh + (h wl + l wh) 2^-32 (+ l wl 2^-64, left out: below half a unit);
-// the middle sum is rounded (the 2^31), so the product is unbiased.
-__device__ __forceinline__ Fix fix_twmul(Fix a, fixw w)
+// the middle sum is rounded (the 2^31).  The product with an exact 1, -1, i or -i
+// ends on a half a quarter of the time, and all of these rounding up would be a
+// drift (at every site where V = 0, and in each stage's first butterfly).  EVEN
+// rounds those of a 1 to even, at two instructions per component; the stage
+// twiddles' tables hold the zero part of such a factor as 2^-62 instead
+// (put_twiddle), so that the sign of the other component decides.
+template <bool EVEN = false> __device__ __forceinline__ Fix fix_twmul(Fix a, fixw w)
 {
     const int xh = fix_hir(a.x), xl = fix_lo(a.x), yh = fix_hir(a.y), yl = fix_lo(a.y);
     const int nh = -w.z, nl = -w.w;
-    long long tr = fix_mad(xh, w.y, 1ll << 31), ti = fix_mad(xh, w.w, 1ll << 31);
+    const long long cr = EVEN ? 0x7fffffffu + (xl & 4) : 0x80000000u, ci = EVEN ? 0x7fffffffu + (yl & 4) : 0x80000000u;
+    long long tr = fix_mad(xh, w.y, cr), ti = fix_mad(xh, w.w, ci);
     tr = fix_mad(xl, w.x, tr);
     ti = fix_mad(xl, w.z, ti);
     tr = fix_mad(yh, nl, tr);
@@ -56,6 +70,26 @@ __device__ __forceinline__ Fix fix_twmul(Fix a, fixw w)
     Fix r;
     r.x = fix_mad(yh, nh, fix_mad(xh, w.x, tr >> 32));
     r.y = fix_mad(yh, w.x, fix_mad(xh, w.z, ti >> 32));
+    return r;
+}
+
+// a w for |a| < 2^61.5: fix_twmul's sums in units four times as fine, with the low
+// words' product, to half a unit
+__device__ __forceinline__ Fix fix_twmul_full(Fix a, fixw w)
+{
+    const int xh = fix_hir(a.x), xl = fix_lo(a.x), yh = fix_hir(a.y), yl = fix_lo(a.y);
+    const int nh = -w.z, nl = -w.w;
+    long long tr = fix_mad(xh, w.y, (1ll << 29) + __mulhi(xl, w.y));
+    long long ti = fix_mad(xh, w.w, (1ll << 29) + __mulhi(xl, w.w));
+    tr = fix_mad(xl, w.x, tr);
+    ti = fix_mad(xl, w.z, ti);
+    tr = fix_mad(yh, nl, tr + __mulhi(yl, nl));
+    ti = fix_mad(yh, w.y, ti + __mulhi(yl, w.y));
+    tr = fix_mad(yl, nh, tr);
+    ti = fix_mad(yl, w.x, ti);
+    Fix r;
+    r.x = fix_mad(yh, nh, fix_mad(xh, w.x, 0)) * 4 + (tr >> 30);
+    r.y = fix_mad(yh, w.x, fix_mad(xh, w.z, 0)) * 4 + (ti >> 30);
     return r;
 }
 
@@ -126,23 +160,23 @@ template <int TL, class Lay, int OP> struct FixReduce {
     }
 };
 
-// the double d as units of 2^(emax - 1023 - 52 - up): its 53-bit significand from bit 52 + up
-// down, shifted by the distance of its exponent from emax (magnitude bits below the unit dropped)
-__device__ __forceinline__ long long fix_from(double d, int emax, int up = 6)
+// the double d as units of 2^(emax - 1023 - 52 - UP): its 53-bit significand from bit 52 + UP
+// down, shifted by the distance of its exponent from emax and rounded to nearest
+template <int UP = 6> __device__ __forceinline__ long long fix_from(double d, int emax)
 {
     const int hi = __double2hiint(d);
     const unsigned lo = (unsigned)__double2loint(d);
     const int e = (hi >> 20) & 0x7ff;
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const unsigned long long m = ((unsigned long long)mh << 32 | lo) << up;
     int sh = emax - e;
     sh = sh > 63 ? 63 : sh;
-    const long long v = (long long)(m >> sh);
+    const unsigned long long m = (((unsigned long long)mh << 32 | lo) << (UP + 1)) >> sh;
     const long long s = (long long)(hi >> 31);
-    return (v ^ s) - s;
+    if constexpr (UP < 10) return (((long long)m ^ s) + 1) >> 1;  // -((m + 1) / 2) = (~m + 1) >> 1
+    return ((long long)((m + 1) >> 1) ^ s) - s;                    // (all 64 bits of m in use)
 }
 
-// v 2^ex as a double, rounded to nearest; ex keeps every result in the normal range (see fix_out)
+// v 2^ex as a double, rounded to nearest (halves away from zero); ex keeps every result in the normal range (see fix_out)
 __device__ __forceinline__ double fix_to(long long v, int ex)
 {
     const int s = fix_hi(v) >> 31;
@@ -222,11 +256,10 @@ template <int E> __device__ __forceinline__ void fix_norm(Fix (&v)[E], unsigned 
     const int top = 31 - __clz((int)m);  // bit length - 1 of the high words (-1: all below 2^32)
     if (top > 28) {
         const int r = top - 28;  // 1 or 2
-        const long long half = 1ll << (r - 1);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            v[e].x = (v[e].x + half) >> r;
-            v[e].y = (v[e].y + half) >> r;
+            v[e].x = fix_shr(v[e].x, r);
+            v[e].y = fix_shr(v[e].y, r);
         }
         ex += r;
     } else if (top < 25) {
@@ -250,7 +283,8 @@ __device__ __forceinline__ bool fix_flagged(const fixw *entry) { return __ldg(&e
 // v 2^ex.  Transforms and unit-modulus products chain without going back to
 // double.  Magnitudes (of the complex values, in units): a transform takes
 // |v| <= 2^59.5 and leaves |v| < 2^63 / sqrt(2); scale() brings components
-// below 2^61; a product takes that and leaves |v| <= 2^59.5.
+// below 2^61; a product takes that and leaves |v| <= 2^59.5; mul_full takes and
+// leaves |v| <= 2^61.5, so another product follows it, or the line's end.
 //
 // Reductions beyond one warp go through four words in the padding of the
 // exchange buffer: word 0 for load(), words 1 .. 3 in turn for the others.  A
@@ -311,12 +345,20 @@ template <int L, int E> struct FixLine {
         fix_norm(v, Red::get(m, w + r), ex);
         if constexpr (!Red::WARP) r = after(r);
     }
-    // v *= f(e); H < E: only the first H slots (the others are not used afterwards)
-    template <int H = E, class F> __device__ __forceinline__ void mul(F f)
+    // v *= f(e); H < E: only the first H slots (the others are not used afterwards).  mul_v: of a
+    // potential table, whose factors may be 1 over most of the line
+    template <int H = E, bool EVEN = false, class F> __device__ __forceinline__ void mul(F f)
     {
 #pragma unroll
-        for (int e = 0; e < H; ++e) v[e] = fix_twmul(v[e], f(e));
+        for (int e = 0; e < H; ++e) v[e] = fix_twmul<EVEN>(v[e], f(e));
         ex += 2;
+    }
+    template <int H = E, class F> __device__ __forceinline__ void mul_v(F f) { mul<H, true>(f); }
+    // the same without the division by four: before another product
+    template <class F> __device__ __forceinline__ void mul_full(F f)
+    {
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = fix_twmul_full(v[e], f(e));
     }
     // The end of a step: the line rounded to doubles and taken up again, as a call that ended
     // here would store it and the next one load it (H < E: slots from H on zero).  A step split
@@ -336,8 +378,8 @@ template <int L, int E> struct FixLine {
     {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            v[e].x = (v[e].x + 2) >> 2;
-            v[e].y = (v[e].y + 2) >> 2;
+            v[e].x = fix_shr(v[e].x, 2);
+            v[e].y = fix_shr(v[e].y, 2);
         }
         ex += 2;
     }
@@ -362,8 +404,8 @@ template <int L, int E> struct FixLine {
             for (int q = 0; q < R; ++q) u[q] = v[j + q * J];
             if constexpr (PP > 1) {
                 const int k = (t + j * TL) & (PP - 1);
-                u[0].x = (u[0].x + 2) >> 2;
-                u[0].y = (u[0].y + 2) >> 2;
+                u[0].x = fix_shr(u[0].x, 2);
+                u[0].y = fix_shr(u[0].y, 2);
 #pragma unroll
                 for (int q = 1; q < R; ++q) u[q] = fix_twmul(u[q], __ldg(&tw[TWO + (q - 1) * PP + k]));
             }

@@ -146,6 +146,9 @@ inline void put_twiddle(int prec, unsigned char *dst, long double re, long doubl
         int32_t v[4];
         put_fixed(re, &v[0], &v[1]);
         put_fixed(im, &v[2], &v[3]);
+        // 1, -1, i, -i: the zero part as the last place (fix_twmul)
+        if ((v[0] | v[1] | v[3]) == 0 && std::abs(v[2]) == 1 << 30) v[1] = 1;
+        if ((v[1] | v[2] | v[3]) == 0 && std::abs(v[0]) == 1 << 30) v[3] = 1;
         std::memcpy(dst, v, 16);
     } else {
         double v[2] = {(double)re, (double)im};

@@ -330,10 +330,10 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
                     }
                     if (vt) {
                         const fixw *vr = opaque(reinterpret_cast<const fixw *>(vt)) + (size_t)row * NY + t;
-                        f.mul([&](int e) { return ld_stream(vr + e * TL); });
+                        f.mul_v([&](int e) { return ld_stream(vr + e * TL); });
                         if (a.vtwice) {
                             f.round(x, sm, lay, lbar, t);
-                            f.mul([&](int e) { return ld_stream(vr + e * TL); });
+                            f.mul_v([&](int e) { return ld_stream(vr + e * TL); });
                         }
                     } else {
                         f.quarter();
@@ -814,10 +814,10 @@ __global__ void __launch_bounds__(W *(N2 / E), W * (N2 / E) <= 256 && (sizeof(T)
                 }
                 if (vt) {
                     const fixw *vr = opaque(vt) + base;
-                    f.mul([&](int e) { return ld_stream(vr + e * stride); });
+                    f.mul_v([&](int e) { return ld_stream(vr + e * stride); });
                     if (a.vtwice) {
                         f.round(x, sm, lay, bar, t);
-                        f.mul([&](int e) { return ld_stream(vr + e * stride); });
+                        f.mul_v([&](int e) { return ld_stream(vr + e * stride); });
                     }
                 } else {
                     f.quarter();
@@ -1069,7 +1069,7 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
         f.load(x, sm, lay, bar, t);
         auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
         if (fix_flagged(tab(v0) - t + L) || (a.order == 4 && fix_flagged(tab(v1) - t + L))) f.finite = false;
-        f.mul([&](int e) { return __ldg(tab(v0) + e * TL); });
+        f.mul_v([&](int e) { return __ldg(tab(v0) + e * TL); });
         for (uint64_t s = 0; s < nsteps; ++s) {
 #pragma unroll 1
             for (int h = 0; h < 2 * nsub; ++h) {
@@ -1082,11 +1082,11 @@ __device__ __forceinline__ void evolve1d_lines(const Evolve1DBatchArgs &a, int f
                     f.ex -= Plan<L, E>::LOGL;  // 1/N
                 else
                     f.conj();
-                f.mul([&](int e) { return __ldg(m + e * TL); });
+                f.mul_v([&](int e) { return __ldg(m + e * TL); });
                 if (kin) f.conj();
                 if (!kin && last && s + 1 < nsteps) {
                     f.round(x, sm, lay, bar, t);
-                    f.mul([&](int e) { return __ldg(m + e * TL); });
+                    f.mul_v([&](int e) { return __ldg(m + e * TL); });
                 }
             }
         }
@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
         f.load(x, sm, lay, bar, t);
         auto tab = [&](const C *p) { return reinterpret_cast<const fixw *>(p) + t; };
         if (fix_flagged(tab(v0) - t + L2 / 2) || (a.order == 4 && fix_flagged(tab(v1) - t + L2 / 2))) f.finite = false;
-        f.template mul<H>([&](int e) { return __ldg(tab(v0) + e * TL); });
+        f.template mul_v<H>([&](int e) { return __ldg(tab(v0) + e * TL); });
         for (uint64_t s = 0; s < nsteps; ++s) {
 #pragma unroll 1
             for (int h = 0; h < 2 * nsub; ++h) {
@@ -1299,10 +1299,10 @@ __global__ void __launch_bounds__(L2 / E) k_evolve1d_wall(Evolve1DBatchArgs a)
                 const bool last = u == nsub - 1, kin = (h & 1) == 0;
                 const fixw *m = tab(kin ? (a.order == 4 && u == 1 ? k1 : k0) : (a.order == 4 && !last ? v1 : v0));
                 if (kin) f.ex -= Plan<L2, E>::LOGL;  // 1/(2N); the table carries the sign
-                f.template mul<H>([&](int e) { return __ldg(m + e * TL); });
+                f.template mul_v<H>([&](int e) { return __ldg(m + e * TL); });
                 if (!kin && last && s + 1 < nsteps) {
                     f.template round<H>(x, sm, lay, bar, t);
-                    f.template mul<H>([&](int e) { return __ldg(m + e * TL); });
+                    f.template mul_v<H>([&](int e) { return __ldg(m + e * TL); });
                 }
             }
         }
