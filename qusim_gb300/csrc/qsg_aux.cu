@@ -235,8 +235,8 @@ __device__ __forceinline__ void reduce_add(double &s, SumF2 &f, C a, const doubl
 }
 
 template <class C, int MODE>
-__global__ void __launch_bounds__(kThreads) k_reduce(const C *__restrict__ psi, const double *__restrict__ V,
-                                                     size_t lo, size_t hi, double *partials)
+__global__ void __launch_bounds__(kThreads) k_reduce(const C *psi, const double *V, size_t lo, size_t hi,
+                                                     double *partials)
 {
     pdl_wait();
     __shared__ double red[32];

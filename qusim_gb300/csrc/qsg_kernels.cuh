@@ -58,7 +58,11 @@ template <> struct PhaseOps<float2> {
 
 template <class C> __device__ __forceinline__ C ld_c(const C *p) { return __ldg(p); }
 // First statement of every kernel that is launched with launch_pdl: waits for
-// the kernels before it on the stream and their writes (see launch_pdl).
+// the kernels before it on the stream and their writes (see launch_pdl).  A load
+// that the compiler may take for invariant is not held behind it, so what a
+// kernel of the stream writes (states, partial sums) is read through plain
+// pointers, without __restrict__ or __ldg, or with ld_stream (volatile assembly);
+// __ldg is for tables, which the host waits for before the first pass reads them.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Streaming loads of psi and of the V tables bypass L1: each element is read
 // once per pass, and letting them allocate evicts the twiddle tables that
