@@ -100,15 +100,13 @@ struct qsg_inst {
     bool wall_ext = false;
     uint64_t n_out = 0;
     // 1D periodic n that is not a power of two: Bluestein transforms of length
-    // blue_m (qsg_blue.cuh); chirp and FFT_M(conj chirp) / M tables, K / n in ktab
+    // blue_m (qsg_blue.cuh); chirp and FFT_M(conj chirp) / M tables, K / n in ktab.
+    // In fixed point (fx) the chirp, hs and K tables of 1D and 2D, with the exponents
+    // of the scaled ones (1D: hs, K / n; 2D: hs of the two sides, the factors along x)
     bool blue = false;
     int blue_m = 0;
     void *bw = nullptr, *bhs = nullptr;
-    // fixed-point forms (fx), and the exponents of the scaled tables (1D: hs, K / n; 2D: hs of
-    // the two sides, the factors along x)
-    void *bwf = nullptr, *bhsf = nullptr;
     int bhs_exp = 0, bk_exp = 0;
-    void *bwxf = nullptr, *bhsxf = nullptr, *bwyf = nullptr, *bhsyf = nullptr;
     int bhsx_exp = 0, bhsy_exp = 0, bkx_exp[2] = {0, 0};
     int bfs_kexp[2] = {0, 0};  // Bluestein four-step: of the two convolution kernels
     // 1D periodic n above the one-CTA Bluestein lengths: Bluestein's convolutions
@@ -394,8 +392,8 @@ int step1d(qsg_inst *in, uint64_t nsteps, int renorm)
         qsg::BlueArgs a{};
         a.psi = in->psi;
         a.tw = in->fx ? in->tw_fx : in->tw;
-        a.w = in->fx ? in->bwf : in->bw;
-        a.hs = in->fx ? in->bhsf : in->bhs;
+        a.w = in->bw;
+        a.hs = in->bhs;
         a.fx = in->fx ? 1 : 0;
         a.hs_exp = in->bhs_exp;
         a.k_exp = in->bk_exp;
@@ -600,8 +598,8 @@ int step2d_blue(qsg_inst *in, uint64_t nsteps, int renorm)
         a.in_k = in_k ? 1 : 0;
         a.out_k = out_k ? 1 : 0;
         a.tw = in->btwy;
-        a.w = in->fx ? in->bwyf : in->bwy;
-        a.hs = in->fx ? in->bhsyf : in->bhsy;
+        a.w = in->bwy;
+        a.hs = in->bhsy;
         a.fx = in->fx ? 1 : 0;
         a.hs_exp = in->bhsy_exp;
         a.nx = in->nx;
@@ -614,8 +612,8 @@ int step2d_blue(qsg_inst *in, uint64_t nsteps, int renorm)
         qsg::Blue2DArgs a{};
         a.psi = in->psi;
         a.tw = in->btwx;
-        a.w = in->fx ? in->bwxf : in->bwx;
-        a.hs = in->fx ? in->bhsxf : in->bhsx;
+        a.w = in->bwx;
+        a.hs = in->bhsx;
         a.fx = in->fx ? 1 : 0;
         a.hs_exp = in->bhsx_exp;
         a.k_exp = in->bkx_exp[d];
@@ -958,6 +956,12 @@ int upload_fixed(qsg_inst *in, const std::vector<std::complex<long double>> &src
     QSG_CUDA(cudaMemcpyAsync(*dst, h.data(), h.size() * 4, cudaMemcpyHostToDevice, in->ctx->st));
     if (exp2) *exp2 = e;
     return QSG_OK;
+}
+
+// in the form of the instance's tables (exp2: of the fixed-point form)
+int upload_table(qsg_inst *in, const std::vector<std::complex<long double>> &src, void **dst, int *exp2 = nullptr)
+{
+    return in->fx ? upload_fixed(in, src, dst, exp2) : upload_factors(in, src, dst);
 }
 
 // --- 1D plans ----------------------------------------------------------------
@@ -1311,21 +1315,14 @@ int build_tables(qsg_inst *in)
                     kt[k][i] *= std::exp(DT * q * tc[k] * (long double)in->dt.imag() / in->hbar);
             }
         }
-        if ((rc = upload_factors(in, w, &in->bw))) return rc;
-        if ((rc = upload_factors(in, hs, &in->bhs))) return rc;
-        if (in->fx) {
-            int we = 0;
-            if ((rc = upload_fixed(in, w, &in->bwf, nullptr))) return rc;
-            if ((rc = upload_fixed(in, hs, &in->bhsf, &in->bhs_exp))) return rc;
+        if ((rc = upload_table(in, w, &in->bw))) return rc;
+        if ((rc = upload_table(in, hs, &in->bhs, &in->bhs_exp))) return rc;
+        for (int k = 0; k < ntab; ++k) {
+            int e = 0;
+            if ((rc = upload_table(in, kt[k], &in->ktab[k], &e))) return rc;
             // (K_0 = 1 in both: one scale)
-            for (int k = 0; k < ntab; ++k) {
-                if ((rc = upload_fixed(in, kt[k], &in->ktab[k], &we))) return rc;
-                if (k > 0 && we != in->bk_exp) return fail(QSG_ERR_STATE, "Bluestein kinetic tables of different scale");
-                in->bk_exp = we;
-            }
-        } else {
-            for (int k = 0; k < ntab; ++k)
-                if ((rc = upload_factors(in, kt[k], &in->ktab[k]))) return rc;
+            if (k > 0 && e != in->bk_exp) return fail(QSG_ERR_STATE, "Bluestein kinetic tables of different scale");
+            in->bk_exp = e;
         }
     } else if (in->dim == 2 && in->blue2) {
         // per side: Bluestein tables; per kinetic coefficient d: exp(a d DTx fold(i)^2) / (nx ny)
@@ -1333,17 +1330,11 @@ int build_tables(qsg_inst *in)
         // src/SplittingMethod2D.cpp:56-79, as a product of the two axes' factors)
         std::vector<std::complex<long double>> w, hs;
         qsg::blue_tables(in->nx, in->bmx, w, hs);
-        if ((rc = upload_factors(in, w, &in->bwx))) return rc;
-        if ((rc = upload_factors(in, hs, &in->bhsx))) return rc;
-        if (in->fx && ((rc = upload_fixed(in, w, &in->bwxf, nullptr)) ||
-                       (rc = upload_fixed(in, hs, &in->bhsxf, &in->bhsx_exp))))
-            return rc;
+        if ((rc = upload_table(in, w, &in->bwx))) return rc;
+        if ((rc = upload_table(in, hs, &in->bhsx, &in->bhsx_exp))) return rc;
         qsg::blue_tables(in->ny, in->bmy, w, hs);
-        if ((rc = upload_factors(in, w, &in->bwy))) return rc;
-        if ((rc = upload_factors(in, hs, &in->bhsy))) return rc;
-        if (in->fx && ((rc = upload_fixed(in, w, &in->bwyf, nullptr)) ||
-                       (rc = upload_fixed(in, hs, &in->bhsyf, &in->bhsy_exp))))
-            return rc;
+        if ((rc = upload_table(in, w, &in->bwy))) return rc;
+        if ((rc = upload_table(in, hs, &in->bhsy, &in->bhsy_exp))) return rc;
         const long double nn = (long double)in->nx * in->ny;
         for (int k = 0; k < ntab; ++k) {
             const long double d = in->order == 2 ? 1.0L : (long double)tc[k];
@@ -1359,8 +1350,7 @@ int build_tables(qsg_inst *in)
                     f[i] = std::complex<long double>(cosl(im), sinl(im)) / (ax == 0 ? nn : 1.0L);
                     if (in->dt.imag() != 0) f[i] *= std::exp(q * (long double)in->dt.imag() / in->hbar);
                 }
-                void **dst = ax == 0 ? &in->bkx[k] : &in->bky[k];
-                rc = in->fx ? upload_fixed(in, f, dst, ax == 0 ? &in->bkx_exp[k] : nullptr) : upload_factors(in, f, dst);
+                rc = ax == 0 ? upload_table(in, f, &in->bkx[k], &in->bkx_exp[k]) : upload_table(in, f, &in->bky[k]);
                 if (rc) return rc;
             }
         }
@@ -2486,6 +2476,7 @@ int qsg_energies(qsg_inst *in, double *kin, double *pot)
                 ba.tw = in->tw;
                 ba.w = in->bw;
                 ba.hs = in->bhs;
+                ba.fx = in->fx ? 1 : 0;
                 ba.n = (int)in->n;
                 ba.wall_n = in->wall_ext ? (int)in->n_out : 0;
                 QSG_CUDA(qsg::launch_kinetic1d_blue(in->prec, in->blue_m, ba, DT, ctx->sums, ctx->st));
@@ -2591,6 +2582,8 @@ int qsg_energies(qsg_inst *in, double *kin, double *pot)
                 a.tw = in->btwy;
                 a.w = in->bwy;
                 a.hs = in->bhsy;
+                a.fx = in->fx ? 1 : 0;
+                a.hs_exp = in->bhsy_exp;
                 a.nx = in->nx;
                 a.ny = in->ny;
                 QSG_CUDA(qsg::launch_row_blue(in->prec, in->bmy, a, ctx->st));

@@ -31,13 +31,16 @@ cudaError_t run_blue(const BlueArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <class T, int M>
+template <class T, int M, bool FX = false>
 cudaError_t run_blue_kin(const BlueArgs &a, double dtk, double *sums, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_blue_kin<T, M, true>(a, dtk, sums, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M);
-    auto k = k_kinetic1d_blue<T, M, E>;
+    auto k = k_kinetic1d_blue<T, M, E, FX>;
     cudaError_t e = prepare_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<1, M / E, smem, st>>>(a, dtk, sums);
@@ -299,25 +302,23 @@ template <class T, int M> constexpr int col_w_of()
     return w < 1 ? 1 : (w > 16 ? 16 : w);
 }
 
-template <class T, int M>
+template <class T, int M, bool FX = false>
 cudaError_t run_col_blue(const Blue2DArgs &a, bool kinetic, double dtx, double dty, double *partials, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8 && !FX) {
+        if (a.fx) return run_col_blue<T, M, true>(a, kinetic, dtx, dty, partials, st);
+    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int W = col_w_of<T, M>();
     const size_t smem = sizeof(cplx_t<T>) * col_tile_elems(sizeof(cplx_t<T>), M, W);
     const unsigned grid = (unsigned)((a.ny + W - 1) / W);
     if (kinetic) {
-        auto k = k_col_blue_kinetic<T, M, E, W>;
+        auto k = k_col_blue_kinetic<T, M, E, W, FX>;
         cudaError_t e = prepare_smem(k, smem);
         if (e != cudaSuccess) return e;
         k<<<grid, W * (M / E), smem, st>>>(a, dtx, dty, partials);
-    } else if (sizeof(T) == 8 && a.fx) {
-        auto k = k_col_blue<T, M, E, W, sizeof(T) == 8>;
-        cudaError_t e = prepare_smem(k, smem);
-        if (e != cudaSuccess) return e;
-        launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a);
     } else {
-        auto k = k_col_blue<T, M, E, W>;
+        auto k = k_col_blue<T, M, E, W, FX>;
         cudaError_t e = prepare_smem(k, smem);
         if (e != cudaSuccess) return e;
         launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a);

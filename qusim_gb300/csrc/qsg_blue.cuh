@@ -204,9 +204,22 @@ __global__ void __launch_bounds__(M / E) k_evolve1d_blue(BlueArgs a)
     }
 }
 
+// Entry i of a factor table in floating point.  FX: of a fixed-point table, each
+// component rounded once to double.
+template <bool FX, class C> __device__ __forceinline__ C ld_factor(const void *tab, int i)
+{
+    if constexpr (FX) {
+        const fixw f = __ldg(static_cast<const fixw *>(tab) + i);
+        return cmk<C>((double)f.x * 0x1p-30 + (double)f.y * 0x1p-62, (double)f.z * 0x1p-30 + (double)f.w * 0x1p-62);
+    } else {
+        return ld_c(static_cast<const C *>(tab) + i);
+    }
+}
+
 // 1D kinetic energy of any length n: one forward DFT of psi, then
-// sums[0] = sum |X_k|^2 fold(k)^2 DT, sums[1] = sum |X_k|^2 over k < n
-template <class T, int M, int E>
+// sums[0] = sum |X_k|^2 fold(k)^2 DT, sums[1] = sum |X_k|^2 over k < n, both
+// times 4^-hs_exp with a fixed-point hs: the energy is their ratio
+template <class T, int M, int E, bool FX = false>
 __global__ void __launch_bounds__(M / E) k_kinetic1d_blue(BlueArgs a, double dtk, double *sums)
 {
     using C = cplx_t<T>;
@@ -218,23 +231,21 @@ __global__ void __launch_bounds__(M / E) k_kinetic1d_blue(BlueArgs a, double dtk
     const int t = threadIdx.x;
     const int n = a.n;
     const C *psi = static_cast<const C *>(a.psi);
-    const C *w = static_cast<const C *>(a.w);
     const RowLayout<PADS> lay{0};
     C x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int j = t + e * TL;
         const bool zero = j >= n || (a.wall_n && (j == 0 || j == a.wall_n));
-        x[e] = zero ? cmk<C>(0, 0) : cmul(psi[j], ld_c(w + j));
+        x[e] = zero ? cmk<C>(0, 0) : cmul(psi[j], ld_factor<FX, C>(a.w, j));
     }
     // FFT -> conj(. hs) -> FFT: X_k = w_k conj(result_k), |X_k| = |result_k|
     const stw_t<C> *tw = static_cast<const stw_t<C> *>(a.tw);
-    const C *hs = static_cast<const C *>(a.hs);
 #pragma unroll 1
     for (int ph = 0; ph < 2; ++ph) {
         if (ph == 1) {
 #pragma unroll
-            for (int e = 0; e < E; ++e) x[e] = cconj(cmul(x[e], ld_c(hs + t + e * TL)));
+            for (int e = 0; e < E; ++e) x[e] = cconj(cmul(x[e], ld_factor<FX, C>(a.hs, t + e * TL)));
         }
         line_fft<C, M, E, false>(x, sm, lay, CtaBarrier{}, t, tw);
     }
@@ -243,7 +254,7 @@ __global__ void __launch_bounds__(M / E) k_kinetic1d_blue(BlueArgs a, double dtk
     for (int e = 0; e < E; ++e) {
         const int k = t + e * TL;
         if (k < n) {
-            const double a2 = abs2d(cmul(cconj(x[e]), ld_c(w + k)));
+            const double a2 = abs2d(cmul(cconj(x[e]), ld_factor<FX, C>(a.w, k)));
             const double f = (double)(k > n / 2 ? n - k : k);
             kin += a2 * f * f * dtk;
             nn += a2;
@@ -290,9 +301,9 @@ struct Blue2DArgs {
 // one DFT of the M-slot line x (zero above the side length): forward when
 // INV is false, the unnormalised inverse otherwise (both through
 // conj(FFT(conj .)) and the one forward transform body)
-template <bool INV, class C, int M, int E, class Lay, class Bar, class TW>
+template <bool INV, class C, int M, int E, bool FX = false, class Lay, class Bar, class TW>
 __device__ __forceinline__ void blue_dft(C (&x)[E], C *sm, const Lay &lay, const Bar &bar, int t, const TW *tw,
-                                         const C *w, const C *hs)
+                                         const void *w, const void *hs)
 {
     constexpr int TL = M / E;
 #pragma unroll 1
@@ -300,17 +311,17 @@ __device__ __forceinline__ void blue_dft(C (&x)[E], C *sm, const Lay &lay, const
         if (ph == 0) {
             // forward: x w; inverse: conj(x) w (the inverse is conj(DFT(conj x)))
 #pragma unroll
-            for (int e = 0; e < E; ++e) x[e] = cmul(INV ? cconj(x[e]) : x[e], ld_c(w + t + e * TL));
+            for (int e = 0; e < E; ++e) x[e] = cmul(INV ? cconj(x[e]) : x[e], ld_factor<FX, C>(w, t + e * TL));
         } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) x[e] = cconj(cmul(x[e], ld_c(hs + t + e * TL)));
+            for (int e = 0; e < E; ++e) x[e] = cconj(cmul(x[e], ld_factor<FX, C>(hs, t + e * TL)));
         }
         line_fft<C, M, E, false>(x, sm, lay, bar, t, tw);
     }
     // forward: X = w conj(y); inverse: conj(w conj(y)) = conj(w) y
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const C wk = ld_c(w + t + e * TL);
+        const C wk = ld_factor<FX, C>(w, t + e * TL);
         x[e] = INV ? cmulc(x[e], wk) : cmul(cconj(x[e]), wk);
     }
 }
@@ -500,7 +511,8 @@ __global__ void __launch_bounds__(W *(M / E), FX && W * (M / E) <= 512 ? 1024 / 
 // Kinetic energy of a 2D grid of any sides: the rows already hold their
 // y-spectra (a forward row pass); forward column DFT, then per CTA
 // partials[2 cta] = sum |X|^2 (fold(kx)^2 DTx + fold(ky)^2 DTy), partials[2 cta + 1] = sum |X|^2
-template <class T, int M, int E, int W>
+// (times 4^-hs_exp with a fixed-point hs)
+template <class T, int M, int E, int W, bool FX = false>
 __global__ void __launch_bounds__(W *(M / E)) k_col_blue_kinetic(Blue2DArgs a, double dtx, double dty,
                                                                   double *partials)
 {
@@ -524,8 +536,7 @@ __global__ void __launch_bounds__(W *(M / E)) k_col_blue_kinetic(Blue2DArgs a, d
         const int i = t + e * TM;
         x[e] = i < nx ? psi[(size_t)i * ny] : cmk<C>(0, 0);
     }
-    blue_dft<false, C, M, E>(x, sm, lay, CtaBarrier{}, t, static_cast<const stw_t<C> *>(a.tw),
-                             static_cast<const C *>(a.w), static_cast<const C *>(a.hs));
+    blue_dft<false, C, M, E, FX>(x, sm, lay, CtaBarrier{}, t, static_cast<const stw_t<C> *>(a.tw), a.w, a.hs);
     double kin = 0, nn = 0;
     const double fy = (double)(col > ny / 2 ? ny - col : col);
 #pragma unroll
