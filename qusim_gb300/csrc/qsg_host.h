@@ -133,6 +133,13 @@ inline void put_fixed(long double v, int32_t *hi, int32_t *lo)
     put_fixed(v1, (double)(v - (long double)v1), hi, lo);
 }
 
+// 1, -1, i, -i as {re hi, re lo, im hi, im lo}: the zero part as the last place (fix_twmul)
+inline void mark_unit(int32_t *v)
+{
+    if ((v[0] | v[1] | v[3]) == 0 && std::abs(v[2]) == 1 << 30) v[1] = 1;
+    if ((v[1] | v[2] | v[3]) == 0 && std::abs(v[0]) == 1 << 30) v[3] = 1;
+}
+
 inline void put_twiddle(int prec, unsigned char *dst, long double re, long double im)
 {
     if (prec == 2) {
@@ -146,9 +153,7 @@ inline void put_twiddle(int prec, unsigned char *dst, long double re, long doubl
         int32_t v[4];
         put_fixed(re, &v[0], &v[1]);
         put_fixed(im, &v[2], &v[3]);
-        // 1, -1, i, -i: the zero part as the last place (fix_twmul)
-        if ((v[0] | v[1] | v[3]) == 0 && std::abs(v[2]) == 1 << 30) v[1] = 1;
-        if ((v[1] | v[2] | v[3]) == 0 && std::abs(v[0]) == 1 << 30) v[3] = 1;
+        mark_unit(v);
         std::memcpy(dst, v, 16);
     } else {
         double v[2] = {(double)re, (double)im};
@@ -209,6 +214,23 @@ struct CircleLD {
             s.push_back(sinl(ang));
         }
     }
+    // theta = 2 pi m / n = k pi / 2 + alpha, alpha = 2 pi a / n with a in [-n/8, n/8); returns k mod 4
+    int quarter(long m, long *a) const
+    {
+        const long n4 = 2 * n8, k = (m + n8) / n4;
+        *a = m - k * n4;
+        return (int)(k & 3);
+    }
+    // cos and -sin of alpha + k pi / 2 from those of alpha
+    template <class V> static void turn(int k, V ca, V sa, V *re, V *im)
+    {
+        switch (k) {
+        case 0: *re = ca; *im = -sa; break;
+        case 1: *re = -sa; *im = -ca; break;
+        case 2: *re = -ca; *im = sa; break;
+        default: *re = sa; *im = ca; break;
+        }
+    }
     void at(long m, long double *re, long double *im) const
     {
         if (!n8) {
@@ -217,18 +239,33 @@ struct CircleLD {
             *im = -sinl(ang);
             return;
         }
-        // theta = 2 pi m / n = k pi / 2 + alpha, alpha = 2 pi a / n with a in [-n/8, n/8)
-        const long n4 = 2 * n8, k = (m + n8) / n4, a = m - k * n4;
-        const long double ca = c[a < 0 ? -a : a], sa = a < 0 ? -s[-a] : s[a];
-        long double cs, sn;
-        switch (k & 3) {
-        case 0: cs = ca; sn = sa; break;
-        case 1: cs = -sa; sn = ca; break;
-        case 2: cs = -ca; sn = -sa; break;
-        default: cs = sa; sn = -ca; break;
+        long a;
+        const int k = quarter(m, &a);
+        turn(k, c[a < 0 ? -a : a], a < 0 ? -s[-a] : s[a], re, im);
+    }
+};
+
+// put_twiddle(3, ...) of the circle's entries, 8 dividing n: the eighth's values
+// are converted once and the symmetries act on the words (the conversion commutes
+// with both), since long double arithmetic is slow where the host has none
+struct CircleFixed {
+    CircleLD circle;
+    std::vector<int32_t> c, s;  // {hi, lo} each
+    explicit CircleFixed(long n) : circle(n), c(2 * circle.c.size()), s(c.size())
+    {
+        for (size_t j = 0; j < circle.c.size(); ++j) {
+            put_fixed(circle.c[j], &c[2 * j], &c[2 * j + 1]);
+            put_fixed(circle.s[j], &s[2 * j], &s[2 * j + 1]);
         }
-        *re = cs;
-        *im = -sn;
+    }
+    void at(long m, int32_t *v) const
+    {
+        long a;
+        const int k = circle.quarter(m, &a);
+        const long j = a < 0 ? -a : a;
+        for (int i = 0; i < 2; ++i)
+            CircleLD::turn(k, c[2 * j + i], a < 0 ? -s[2 * j + i] : s[2 * j + i], &v[i], &v[2 + i]);
+        mark_unit(v);
     }
 };
 
@@ -271,13 +308,20 @@ inline int get_fs_grid(qsg_ctx *ctx, int prec, int n1, int n2, const void **out)
     }
     const long n = (long)n1 * n2;
     std::vector<unsigned char> host((size_t)n * twsize(prec));
-    const CircleLD circle(n);
-    for (long r = 0; r < n2; ++r)
-        for (long c = 0; c < n1; ++c) {
-            long double re, im;
-            circle.at(r * c, &re, &im);
-            put_twiddle(prec, &host[(size_t)(r * n1 + c) * twsize(prec)], re, im);
-        }
+    if (prec == 3 && n % 8 == 0) {
+        const CircleFixed circle(n);
+        int32_t *v = reinterpret_cast<int32_t *>(host.data());
+        for (long r = 0; r < n2; ++r)
+            for (long c = 0; c < n1; ++c, v += 4) circle.at(r * c, v);
+    } else {
+        const CircleLD circle(n);
+        for (long r = 0; r < n2; ++r)
+            for (long c = 0; c < n1; ++c) {
+                long double re, im;
+                circle.at(r * c, &re, &im);
+                put_twiddle(prec, &host[(size_t)(r * n1 + c) * twsize(prec)], re, im);
+            }
+    }
     void *d = nullptr;
     int rc = dev_alloc(ctx, host.size(), &d, nullptr);
     if (rc) return rc;
