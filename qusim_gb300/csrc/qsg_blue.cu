@@ -6,46 +6,13 @@
 #include <thread>
 #include <vector>
 
-#include "qsg_blue.cuh"
-#include "qsg_dispatch.cuh"
+#include "qsg_blue_inst.cuh"
 
 namespace qsg {
 
 namespace {
 
 constexpr int blue_e(int prec) { return prec == 1 ? 16 : 8; }
-
-template <class T, int M, bool FX = false>
-cudaError_t run_blue(const BlueArgs &a, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_blue<T, M, true>(a, st);
-    }
-    constexpr int E = FX ? blue_fx_e(M) : (sizeof(T) == 4 ? 16 : 8);
-    constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
-    const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M);
-    auto k = k_evolve1d_blue<T, M, E, FX>;
-    cudaError_t e = prepare_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3(1), dim3(M / E), smem, st, a);
-    return cudaGetLastError();
-}
-
-template <class T, int M, bool FX = false>
-cudaError_t run_blue_kin(const BlueArgs &a, double dtk, double *sums, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_blue_kin<T, M, true>(a, dtk, sums, st);
-    }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
-    constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
-    const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M);
-    auto k = k_kinetic1d_blue<T, M, E, FX>;
-    cudaError_t e = prepare_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    k<<<1, M / E, smem, st>>>(a, dtk, sums);
-    return cudaGetLastError();
-}
 
 // in-place forward DFT of a power-of-two length in long double (iterative
 // radix 2, twiddles from cosl / sinl of the exact angle)
@@ -248,11 +215,12 @@ void blue_tables_dd(uint64_t n, uint64_t m, std::vector<std::complex<double>> &w
 
 cudaError_t launch_evolve1d_blue(int prec, int m, const BlueArgs &a, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_evolve1d_blue_fx(m, a, st);
 #define X(T, M) case M: return run_blue<T, M>(a, st);
     if (prec == 1) {
-        switch (m) { X(float, 256) X(float, 512) X(float, 1024) X(float, 2048) X(float, 4096) X(float, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, float) default: break; }
     } else {
-        switch (m) { X(double, 256) X(double, 512) X(double, 1024) X(double, 2048) X(double, 4096) X(double, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, double) default: break; }
     }
 #undef X
     return cudaErrorNotSupported;
@@ -260,11 +228,12 @@ cudaError_t launch_evolve1d_blue(int prec, int m, const BlueArgs &a, cudaStream_
 
 cudaError_t launch_kinetic1d_blue(int prec, int m, const BlueArgs &a, double dtk, double *sums, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_kinetic1d_blue_fx(m, a, dtk, sums, st);
 #define X(T, M) case M: return run_blue_kin<T, M>(a, dtk, sums, st);
     if (prec == 1) {
-        switch (m) { X(float, 256) X(float, 512) X(float, 1024) X(float, 2048) X(float, 4096) X(float, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, float) default: break; }
     } else {
-        switch (m) { X(double, 256) X(double, 512) X(double, 1024) X(double, 2048) X(double, 4096) X(double, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, double) default: break; }
     }
 #undef X
     return cudaErrorNotSupported;
@@ -277,64 +246,14 @@ int blue_elems(int prec) { return blue_e(prec); }
 int blue_rows_per_cta(int prec, int m) { return std::max(1, 256 / (m / blue_e(prec))); }
 int blue_cols_per_cta(int prec, int m) { return std::max(1, std::min(16, 65536 / (m * (prec == 1 ? 8 : 16)))); }
 
-namespace {
-
-template <class T, int M, bool FX = false>
-cudaError_t run_row_blue(const Blue2DArgs &a, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_row_blue<T, M, true>(a, st);
-    }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
-    constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
-    constexpr int RPC = (256 / (M / E)) > 1 ? 256 / (M / E) : 1;
-    const size_t smem = sizeof(cplx_t<T>) * padded<M, PADS>(M) * RPC;
-    auto k = k_row_blue<T, M, E, RPC, FX>;
-    cudaError_t e = prepare_smem(k, smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3((a.nx + RPC - 1) / RPC), dim3(RPC * (M / E)), smem, st, a);
-    return cudaGetLastError();
-}
-
-template <class T, int M> constexpr int col_w_of()
-{
-    constexpr int w = 65536 / (M * (int)sizeof(cplx_t<T>));
-    return w < 1 ? 1 : (w > 16 ? 16 : w);
-}
-
-template <class T, int M, bool FX = false>
-cudaError_t run_col_blue(const Blue2DArgs &a, bool kinetic, double dtx, double dty, double *partials, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_col_blue<T, M, true>(a, kinetic, dtx, dty, partials, st);
-    }
-    constexpr int E = sizeof(T) == 4 ? 16 : 8;
-    constexpr int W = col_w_of<T, M>();
-    const size_t smem = sizeof(cplx_t<T>) * col_tile_elems(sizeof(cplx_t<T>), M, W);
-    const unsigned grid = (unsigned)((a.ny + W - 1) / W);
-    if (kinetic) {
-        auto k = k_col_blue_kinetic<T, M, E, W, FX>;
-        cudaError_t e = prepare_smem(k, smem);
-        if (e != cudaSuccess) return e;
-        k<<<grid, W * (M / E), smem, st>>>(a, dtx, dty, partials);
-    } else {
-        auto k = k_col_blue<T, M, E, W, FX>;
-        cudaError_t e = prepare_smem(k, smem);
-        if (e != cudaSuccess) return e;
-        launch_pdl(k, dim3(grid), dim3(W * (M / E)), smem, st, a);
-    }
-    return cudaGetLastError();
-}
-
-}  // namespace
-
 cudaError_t launch_row_blue(int prec, int m, const Blue2DArgs &a, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_row_blue_fx(m, a, st);
 #define X(T, MM) case MM: return run_row_blue<T, MM>(a, st);
     if (prec == 1) {
-        switch (m) { X(float, 256) X(float, 512) X(float, 1024) X(float, 2048) X(float, 4096) X(float, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, float) default: break; }
     } else {
-        switch (m) { X(double, 256) X(double, 512) X(double, 1024) X(double, 2048) X(double, 4096) X(double, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, double) default: break; }
     }
 #undef X
     return cudaErrorNotSupported;
@@ -343,11 +262,12 @@ cudaError_t launch_row_blue(int prec, int m, const Blue2DArgs &a, cudaStream_t s
 cudaError_t launch_col_blue(int prec, int m, const Blue2DArgs &a, bool kinetic, double dtx, double dty,
                             double *partials, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_col_blue_fx(m, a, kinetic, dtx, dty, partials, st);
 #define X(T, MM) case MM: return run_col_blue<T, MM>(a, kinetic, dtx, dty, partials, st);
     if (prec == 1) {
-        switch (m) { X(float, 256) X(float, 512) X(float, 1024) X(float, 2048) X(float, 4096) X(float, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, float) default: break; }
     } else {
-        switch (m) { X(double, 256) X(double, 512) X(double, 1024) X(double, 2048) X(double, 4096) X(double, 8192) default: break; }
+        switch (m) { QSG_BLUE_M(X, double) default: break; }
     }
 #undef X
     return cudaErrorNotSupported;

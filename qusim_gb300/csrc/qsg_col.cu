@@ -63,7 +63,9 @@ extern template cudaError_t launch_row_pass_f32a_t<false>(const Geom2D &, const 
 extern template cudaError_t launch_row_pass_f32a_t<true>(const Geom2D &, const RowPassArgs &, cudaStream_t);
 extern template cudaError_t launch_row_pass_f32b_t<false>(const Geom2D &, const RowPassArgs &, cudaStream_t);
 extern template cudaError_t launch_row_pass_f32b_t<true>(const Geom2D &, const RowPassArgs &, cudaStream_t);
-cudaError_t launch_row_pass_f64(const Geom2D &, const RowPassArgs &, cudaStream_t);
+template <bool FX> cudaError_t launch_row_pass_f64_t(const Geom2D &, const RowPassArgs &, cudaStream_t);
+extern template cudaError_t launch_row_pass_f64_t<false>(const Geom2D &, const RowPassArgs &, cudaStream_t);
+extern template cudaError_t launch_row_pass_f64_t<true>(const Geom2D &, const RowPassArgs &, cudaStream_t);
 bool row_variant_exists_f32a(int ny, int e, int g, int nt);
 bool row_variant_exists_f32b(int ny, int e, int g, int nt);
 bool row_variant_exists_f64(int ny, int e, int g, int nt);
@@ -71,7 +73,7 @@ bool row_variant_exists_f64(int ny, int e, int g, int nt);
 cudaError_t launch_row_pass(int prec, const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
 {
     if (g.row_kind == 1) return launch_row_pass_tm(g, a, st);
-    if (prec == 0) return launch_row_pass_f64(g, a, st);
+    if (prec == 0) return a.fx ? launch_row_pass_f64_t<true>(g, a, st) : launch_row_pass_f64_t<false>(g, a, st);
     if (g.row_e == 16) return a.plain ? launch_row_pass_f32a_t<true>(g, a, st) : launch_row_pass_f32a_t<false>(g, a, st);
     return a.plain ? launch_row_pass_f32b_t<true>(g, a, st) : launch_row_pass_f32b_t<false>(g, a, st);
 }

@@ -53,6 +53,7 @@ cudaError_t launch_evolve1d(int prec, int n, const Evolve1DBatchArgs &a, cudaStr
 {
     const bool few = n >= 64 && res_few(n, prec == 1 ? 16 : 8, a.count);
     if (prec == 1 && few) return launch_evolve1d_few_f32(n, a, st);
+    if (prec == 0 && a.fx) return launch_evolve1d_fx(n, few, a, st);
 #define X(T, L) case L: return run_evolve1d<T, L, false>(a, st);
 #define Y(T, L) case L: return run_evolve1d<T, L, true>(a, st);
     if (prec == 1) {
@@ -106,6 +107,7 @@ static cudaError_t run_wallkin(const void *psi, const void *tw, double dtk, doub
 cudaError_t launch_wall1d(int prec, int n, const Evolve1DBatchArgs &a, cudaStream_t st)
 {
     if (prec == 1) return launch_wall1d_f32(n, a, st);
+    if (a.fx) return launch_wall1d_fx(n, a, st);
 #define X(T, L) case L / 2: return run_wall<T, L>(a, st);
     switch (n) { QSG_1D_CASES(X, double) default: break; }
 #undef X
@@ -131,12 +133,6 @@ cudaError_t launch_kinetic1d_wall(int prec, int n, const void *psi, const void *
 // where that would make n2 2048 (a column pass of 2048-point columns takes two
 // columns per CTA: 16-byte row segments, half a memory sector)
 // ---------------------------------------------------------------------------
-
-constexpr int fs_col_w(int prec, int n2) { return prec == 1 ? 4096 / n2 : 2048 / n2; }   // W*n2/E = 256
-constexpr int fs_row_b(int prec, int n1)   // B*n1/E = 256 (512 for complex128 rows of 4096)
-{
-    return prec == 1 ? 4096 / n1 : (n1 >= 2048 ? 1 : 2048 / n1);
-}
 
 int fs_default_n1(uint64_t n)
 {
@@ -172,38 +168,6 @@ bool fs_geom(int prec, uint64_t n, FsGeom *g, int n1)
     return g->col_blocks >= 1 && g->row_blocks >= 1;
 }
 
-template <class T, int N2, bool FX = false>
-static cudaError_t run_fs_col(const FsGeom &g, const FsColArgs &a, int ninst, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_fs_col<T, N2, true>(g, a, ninst, st);
-    }
-    constexpr int P = sizeof(T) == 4 ? 1 : 0;
-    constexpr int E = P ? 16 : 8;
-    constexpr int W = fs_col_w(P, N2);
-    auto k = k_fs_col<T, N2, E, W, FX>;
-    cudaError_t e = prepare_smem(k, g.col_smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3(g.col_blocks, ninst), dim3(W * (N2 / E)), g.col_smem, st, a);
-    return cudaGetLastError();
-}
-
-template <class T, int N1, bool FX = false>
-static cudaError_t run_fs_row(const FsGeom &g, const FsRowArgs &a, int ninst, cudaStream_t st)
-{
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_fs_row<T, N1, true>(g, a, ninst, st);
-    }
-    constexpr int P = sizeof(T) == 4 ? 1 : 0;
-    constexpr int E = P ? 16 : 8;
-    constexpr int B = fs_row_b(P, N1);
-    auto k = k_fs_row<T, N1, E, B, FX>;
-    cudaError_t e = prepare_smem(k, g.row_smem);
-    if (e != cudaSuccess) return e;
-    launch_pdl(k, dim3(g.row_blocks, ninst), dim3(B * (N1 / E)), g.row_smem, st, a);
-    return cudaGetLastError();
-}
-
 template <class T, int N1>
 static cudaError_t run_fs_rowkin(const FsGeom &g, const FsRowArgs &a, double dtk, double *partials,
                                  cudaStream_t st)
@@ -218,11 +182,9 @@ static cudaError_t run_fs_rowkin(const FsGeom &g, const FsRowArgs &a, double dtk
     return cudaGetLastError();
 }
 
-#define QSG_FS_N(X, T) X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048) X(T, 4096)
-#define QSG_FS_N2(X, T) X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048)
-
 cudaError_t launch_fs_col(int prec, const FsGeom &g, const FsColArgs &a, int ninst, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_fs_col_fx(g, a, ninst, st);
 #define X(T, N2) case N2: return run_fs_col<T, N2>(g, a, ninst, st);
     if (prec == 1) {
         switch (g.n2) { QSG_FS_N2(X, float) default: break; }
@@ -235,6 +197,7 @@ cudaError_t launch_fs_col(int prec, const FsGeom &g, const FsColArgs &a, int nin
 
 cudaError_t launch_fs_row(int prec, const FsGeom &g, const FsRowArgs &a, int ninst, cudaStream_t st)
 {
+    if (prec == 0 && a.fx) return launch_fs_row_fx(g, a, ninst, st);
 #define X(T, N1) case N1: return run_fs_row<T, N1>(g, a, ninst, st);
     if (prec == 1) {
         switch (g.n1) { QSG_FS_N(X, float) default: break; }

@@ -1,5 +1,6 @@
 // qsg_evolve1d_inst.cuh -- launchers of the one-CTA 1D kernels, instantiated by
-// qsg_evolve1d.cu and qsg_evolve1d_f32.cu (packed pairs).
+// qsg_evolve1d.cu, qsg_evolve1d_f32.cu (packed pairs) and qsg_evolve1d_fx.cu (complex128 in
+// fixed point), and of the four-step passes.
 #pragma once
 #include "qsg_dispatch.cuh"
 
@@ -21,9 +22,6 @@ static inline bool res_few(int l, int e, int count) { return count <= res_ni_for
 template <class T, int L, bool FEW, bool FX = false>
 static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
 {
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_evolve1d<T, L, FEW, true>(a, st);
-    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     constexpr int NI = res_ni_for(L, E, FEW);
@@ -38,9 +36,6 @@ static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
 template <class T, int L2, bool FX = false>
 static cudaError_t run_wall(const Evolve1DBatchArgs &a, cudaStream_t st)
 {
-    if constexpr (sizeof(T) == 8 && !FX) {
-        if (a.fx) return run_wall<T, L2, true>(a, st);
-    }
     constexpr int E = sizeof(T) == 4 ? 16 : 8;
     constexpr int PADS = sizeof(T) == 4 ? 4 : 3;
     const size_t smem = sizeof(cplx_t<T>) * padded<L2, PADS>(L2);
@@ -51,7 +46,47 @@ static cudaError_t run_wall(const Evolve1DBatchArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// four-step passes: columns per column-pass CTA, rows per row-pass CTA
+constexpr int fs_col_w(int prec, int n2) { return prec == 1 ? 4096 / n2 : 2048 / n2; }   // W*n2/E = 256
+constexpr int fs_row_b(int prec, int n1)   // B*n1/E = 256 (512 for complex128 rows of 4096)
+{
+    return prec == 1 ? 4096 / n1 : (n1 >= 2048 ? 1 : 2048 / n1);
+}
+
+template <class T, int N2, bool FX = false>
+static cudaError_t run_fs_col(const FsGeom &g, const FsColArgs &a, int ninst, cudaStream_t st)
+{
+    constexpr int P = sizeof(T) == 4 ? 1 : 0;
+    constexpr int E = P ? 16 : 8;
+    constexpr int W = fs_col_w(P, N2);
+    auto k = k_fs_col<T, N2, E, W, FX>;
+    cudaError_t e = prepare_smem(k, g.col_smem);
+    if (e != cudaSuccess) return e;
+    launch_pdl(k, dim3(g.col_blocks, ninst), dim3(W * (N2 / E)), g.col_smem, st, a);
+    return cudaGetLastError();
+}
+
+template <class T, int N1, bool FX = false>
+static cudaError_t run_fs_row(const FsGeom &g, const FsRowArgs &a, int ninst, cudaStream_t st)
+{
+    constexpr int P = sizeof(T) == 4 ? 1 : 0;
+    constexpr int E = P ? 16 : 8;
+    constexpr int B = fs_row_b(P, N1);
+    auto k = k_fs_row<T, N1, E, B, FX>;
+    cudaError_t e = prepare_smem(k, g.row_smem);
+    if (e != cudaSuccess) return e;
+    launch_pdl(k, dim3(g.row_blocks, ninst), dim3(B * (N1 / E)), g.row_smem, st, a);
+    return cudaGetLastError();
+}
+
+#define QSG_FS_N(X, T) X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048) X(T, 4096)
+#define QSG_FS_N2(X, T) X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048)
+
 cudaError_t launch_evolve1d_few_f32(int n, const Evolve1DBatchArgs &a, cudaStream_t st);
 cudaError_t launch_wall1d_f32(int n, const Evolve1DBatchArgs &a, cudaStream_t st);
+cudaError_t launch_evolve1d_fx(int n, bool few, const Evolve1DBatchArgs &a, cudaStream_t st);
+cudaError_t launch_wall1d_fx(int n, const Evolve1DBatchArgs &a, cudaStream_t st);
+cudaError_t launch_fs_col_fx(const FsGeom &g, const FsColArgs &a, int ninst, cudaStream_t st);
+cudaError_t launch_fs_row_fx(const FsGeom &g, const FsRowArgs &a, int ninst, cudaStream_t st);
 
 }  // namespace qsg

@@ -1,4 +1,5 @@
-// 2D row passes (double): instantiations + launcher.
+// 2D row passes (double): instantiations + launchers, fixed-point products here and
+// double ones (complex time steps) in qsg_row_f64_double.cu, which includes this.
 #include "qsg_dispatch.cuh"
 
 namespace qsg {
@@ -17,15 +18,17 @@ static cudaError_t run_row_f64(const Geom2D &g, const RowPassArgs &a, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launch_row_pass_f64(const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
+template <bool FX> cudaError_t launch_row_pass_f64_t(const Geom2D &g, const RowPassArgs &a, cudaStream_t st)
 {
 #define X(T, NY, E, G, NT) \
-    if (g.ny == NY && g.row_e == E && g.g == G && g.row_threads == NT) \
-        return a.fx ? run_row_f64<NY, E, G, NT, true>(g, a, st) : run_row_f64<NY, E, G, NT, false>(g, a, st);
+    if (g.ny == NY && g.row_e == E && g.g == G && g.row_threads == NT) return run_row_f64<NY, E, G, NT, FX>(g, a, st);
     QSG_ROW_VARIANTS_F64(X)
 #undef X
     return cudaErrorNotSupported;
 }
+
+#ifndef QSG_DOUBLE_UNIT
+template cudaError_t launch_row_pass_f64_t<true>(const Geom2D &, const RowPassArgs &, cudaStream_t);
 
 bool row_variant_exists_f64(int ny, int e, int g, int nt)
 {
@@ -35,5 +38,9 @@ bool row_variant_exists_f64(int ny, int e, int g, int nt)
 #undef X
     return false;
 }
+
+#else
+template cudaError_t launch_row_pass_f64_t<false>(const Geom2D &, const RowPassArgs &, cudaStream_t);
+#endif
 
 }  // namespace qsg
