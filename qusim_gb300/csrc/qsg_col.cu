@@ -156,7 +156,7 @@ int candidate_plans(int prec, int nx, int ny, Plan2D *out, int cap)
 bool default_plan(int prec, int nx, int ny, Plan2D *p)
 {
     // complex64: column blocks of <= 1024 rows with 64-byte column segments
-    // (radix 16); complex128: blocks of <= 2048 rows (radix 8)
+    // (radix 16 and 32); complex128: unsplit columns of up to 4096 rows (radix 8)
     Plan2D c;
     if (prec == 1) {
         c.g = nx > 1024 ? nx / 1024 : 1;
@@ -168,17 +168,16 @@ bool default_plan(int prec, int nx, int ny, Plan2D *p)
         // radix 32: two stages (one exchange) for 512- and 1024-point columns
         if (m == 1024) c.col_e = 32;
         if (m == 512) {
-            c.col_e = 32;
-            c.col_w = 16;
+            // 16 columns per CTA where they make 128 tiles (512 x 2048: 47.0 us an O4 step, 54.1 with
+            // 256 tiles of 8 columns in radix 8); fewer leave SMs idle (512 x 1024: 36.6 with 64 tiles,
+            // 30.6 with 128 of 8 columns)
+            const bool fill = c.g * ny / 16 >= 128;
+            c.col_e = fill ? 32 : 8;
+            c.col_w = fill ? 16 : 8;
         }
         // unsplit rows of 1024 and 2048 points: units of two rows and one, which fill
         // the SMs more evenly (1024^2 48.4 -> 46.4 us, 1024 x 2048 87.5 -> 81.0)
         if (c.g == 1 && (ny == 1024 || ny == 2048)) c.row_nt = 128;
-        // (512 x 1024: radix-8 columns fill the chip too, 38.4 -> 30.9 us)
-        if (nx == 512 && ny == 1024) {
-            c.col_e = 8;
-            c.col_w = 8;
-        }
         // Small grids leave lanes idle and are bound by the instructions one
         // thread runs in a row: radix 8 (twice the threads), shorter columns, fewer
         // columns per CTA.  Per O4 step against the rule above: 128^2 16.5 / 23.5
