@@ -197,18 +197,19 @@ bool default_plan(int prec, int nx, int ny, Plan2D *p)
         }
     } else {
         // the x split's stages would run in FP64 (2 instructions per clock): only
-        // the 8192-row grids, whose columns do not fit a CTA, take one (4096^2:
-        // 714 + 595 us a column and a row pass unsplit, 570 + 860 split in two).
+        // the 8192-row grids, whose columns do not fit a CTA, take one (O4 step of
+        // 4096^2 unsplit 4.04 ms, split in two 4.43; 4096 x 2048 1.91 / 2.10, x 512
+        // 0.47 / 0.48, x 256 0.25 / 0.27; x 1024 1.02 / 0.96 and x 128, 64 tiles,
+        // 0.21 / 0.16 are better split, and left to the tuner).
         c.g = nx > 4096 ? nx / 2048 : 1;
         const int m = nx / c.g;
         // Small grids are bound by the instructions one thread runs in a row: four
-        // elements a thread instead of eight (128 x 128: 10.2 against 12.4 us a
-        // pass; at 512^2 the chip is full and eight win, 15.9 + 14.5 against
-        // 18.6 + 16.2).
+        // elements a thread instead of eight (O4 step of 128 x 128: 36.4 against 52.2
+        // us; at 512^2 the chip is full and eight win, 67.7 against 76.8).
         const bool small = (long)nx * ny <= 65536 && m <= 256 && ny <= 256 && c.g == 1;
         c.row_e = small ? 4 : 8;
-        // the fewest threads that hold whole rows: more, shorter units (1024^2: 35.6
-        // with 128 threads against 41.0 us with 256)
+        // the fewest threads that hold whole rows: more, shorter units (O4 step of
+        // 1024^2: 232 us with 128 threads, 240 with 256)
         const int tl = ny / c.row_e;
         c.row_nt = c.g > 1 ? (row_work_for(ny, 8, c.g, 256) >= 512 ? 512 : 256) : small ? 128 : (tl > 64 ? tl : 64);
         c.col_e = small ? 4 : 8;

@@ -1,8 +1,8 @@
 // One-CTA 1D evolution in complex64 where a launch has at most a CTA per SM (a
 // line of its own, small batches), and walls.  Packed FP32 pairs: a CTA alone on
 // its SM has the registers (up to 244 per thread), and its step is bound by the
-// instructions it issues (n = 4096 O2: 4.43 -> 3.35 us a step, n = 1024: 3.42 ->
-// 2.67).  Launches over more lines, the tile queue and the four-step passes stay
+// instructions it issues (with the CTAs of one line, per O2 step: n = 64 1.84 ->
+// 1.27 us, 1024 3.35 -> 1.53, 4096 4.36 -> 3.28).  Launches over more lines, the tile queue and the four-step passes stay
 // scalar in qsg_evolve1d.cu: under their register caps the pairs spill (queue of
 // 256 .. 2048-site lines 614 -> 1122 us per 100 steps).  Both round alike.
 #define QSG_PACKED_F32

@@ -449,9 +449,9 @@ template <int L, int E> struct FixLine {
 };
 
 // Forward transform of a complex128 line (line_fft's contract).
-// Measured against FP64 butterflies (whole calls): 1024^2 O4 1035 -> 332 us a
-// step, a 1000-site wall 595 -> 204 us, 131072-site lines 82 -> 41 us, 450 x 700
-// 668 -> 247 us.
+// Per step against FP64 butterflies and products, with the chained passes and the
+// plans that came with them: 1024^2 O4 1026 -> 235 us, a 1000-site wall 593 -> 122,
+// a 131072-site line (O2) 79.8 -> 25.8, 450 x 700 1991 -> 438.
 template <int L, int E, class Lay, class Bar>
 __device__ __forceinline__ void line_fft_fix(double2 (&x)[E], double2 *smd, const Lay &lay, const Bar &bar, int t,
                                              const fixw *__restrict__ tw)

@@ -192,9 +192,9 @@ template <class C, bool PL> using pass_stw_t = std::conditional_t<PL, float2, st
 
 // FX (complex128 with a real time step, so unit-modulus factors): a line goes
 // to fixed point once, runs transform, potential product and transform there,
-// and comes back once (1024^2, with the plans of shorter units: 53 -> 40 us a
-// row pass, 60 -> 44 us a column pass; the line's rounding at a step's end,
-// FixLine::round, is 4 of the 40).
+// and comes back once (1024^2, with the plans of shorter units: 53 -> 39 us a
+// row pass, 46 where a step ends, with V twice and FixLine::round between; 60 ->
+// 42 us a column pass).
 template <class T, int NY, int E, int G, int B, int RS, bool IN, bool PL, bool FX>
 __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned char *smraw, double *red)
 {
@@ -443,8 +443,8 @@ __device__ __forceinline__ void row_pass_units(const RowPassArgs &a, unsigned ch
 // One kernel serves the three pass kinds of a step (runtime flags); the body
 // is specialised on in_split so that the registers holding the next unit's
 // input exist only where that input is split-k.
-// complex128 runs at three CTAs of 256 threads per SM (85 registers): with two
-// (126) its integer pipes wait more (1024^2: 51.5 -> 43.3 us per launch).
+// complex128 runs 768 threads per SM (85 registers): with 512 its integer pipes
+// wait more (1024^2: 41.0 -> 39.4 us per launch).
 template <class T, int NY, int E, int G, int B, int RS, bool PL = false, bool FX = false>
 __global__ void __launch_bounds__(B *G *(NY / E) / RS, sizeof(T) == 8 ? (G == 1 ? 768 : 512) / (B * G * (NY / E) / RS) : 0)
     k_row_pass(RowPassArgs a)
@@ -484,8 +484,8 @@ struct ColPassArgs {
 // Radix-32 variants are held to 128 registers so that 512 threads (two CTAs
 // of 256) share an SM.  (Four CTAs of 128 threads, W = 4, measured slower at
 // 4096^2: 168 against 119 us.)
-// complex128 is held to 64 registers (1024 threads per SM): 1024^2 60.3 -> 52.0
-// us per launch with four columns, 2048^2 209 -> 169 us with two.
+// complex128 is held to 64 registers (1024 threads per SM): 1024^2, two columns,
+// 43.8 -> 42.4 us per launch against 512 threads.
 template <class T, int M, int E, int W, bool PL = false, bool FX = false>
 __global__ void __launch_bounds__(W *(M / E), E == 32 ? 512 / (W * (M / E)) : sizeof(T) == 8 ? 1024 / (W * (M / E)) : 1)
     k_col_pass(ColPassArgs a)

@@ -32,10 +32,8 @@ int blue_m_for(int prec, uint64_t n);
 int blue_elems(int prec);
 // elements per thread of the 1D fixed-point kernel (complex128, real time steps):
 // four, twice the warps, up to M = 1024, where one CTA's line leaves its SM idle
-// (per O4 step n = 100 29.5 -> 20.9 us, 200 32.2 -> 27.7, 500 42.4 -> 40.6);
-// above, eight with fewer stages (n = 1000 63.0 against 81.3 with four).  The
-// rounding at a step's end has since added 1.2 us (n = 100) to 3.6 us (n = 1000)
-// to each of these
+// (per O4 step n = 100 33.6 -> 22.1 us, 200 37.3 -> 29.2, 500 50.3 -> 41.9);
+// above, eight with fewer stages (n = 1000 67.0 against 82.5 with four)
 constexpr int blue_fx_e(int m) { return m <= 1024 ? 4 : 8; }
 void blue_tables(uint64_t n, int m, std::vector<std::complex<long double>> &w,
                  std::vector<std::complex<long double>> &hs);
