@@ -106,10 +106,13 @@ static cudaError_t run_wallkin(const void *psi, const void *tw, double dtk, doub
 
 cudaError_t launch_wall1d(int prec, int n, const Evolve1DBatchArgs &a, cudaStream_t st)
 {
-    if (prec == 1) return launch_wall1d_f32(n, a, st);
-    if (a.fx) return launch_wall1d_fx(n, a, st);
+    if (prec == 0 && a.fx) return launch_wall1d_fx(n, a, st);
 #define X(T, L) case L / 2: return run_wall<T, L>(a, st);
-    switch (n) { QSG_1D_CASES(X, double) default: break; }
+    if (prec == 1) {
+        switch (n) { QSG_WALL_SCALAR(X, float) default: return launch_wall1d_f32(n, a, st); }
+    } else {
+        switch (n) { QSG_1D_CASES(X, double) default: break; }
+    }
 #undef X
     return cudaErrorNotSupported;
 }

@@ -19,6 +19,13 @@ static inline bool res_few(int l, int e, int count) { return count <= res_ni_for
 #define QSG_1D_CASES(X, T) \
     X(T, 64) X(T, 128) X(T, 256) X(T, 512) X(T, 1024) X(T, 2048) X(T, 4096)
 
+// complex64 walls (lines of L = 2n): in packed pairs where the last stage is of
+// radix 4 or 8, scalar where all stages are of radix 16 (and one of 2).  Scalar to
+// packed, us per O4 step: n = 64 4.10 -> 3.83, 512 5.99 -> 5.72, 1024 7.47 -> 7.04;
+// 128 3.99 -> 4.26, 256 5.84 -> 6.00, 2048 11.29 -> 11.77, 4096 31.3 -> 31.8.
+#define QSG_WALL_PACKED(X, T) X(T, 128) X(T, 1024) X(T, 2048)
+#define QSG_WALL_SCALAR(X, T) X(T, 256) X(T, 512) X(T, 4096) X(T, 8192)
+
 template <class T, int L, bool FEW, bool FX = false>
 static cudaError_t run_evolve1d(const Evolve1DBatchArgs &a, cudaStream_t st)
 {
